@@ -77,15 +77,48 @@ template <class RL> __device__ __forceinline__ int pidx(int e) {
     return padi(e);
 }
 
+// Slots of a butterfly's elements e0 + r*ST.  Where the pad of those elements
+// differs from e0's by a constant, the slot is pidx(e0) plus a compile-time
+// offset (one address per butterfly, immediate offsets in the accesses)
+// instead of an add, a shift and an add per element:
+//   reads  (ST = nb = L/RAD, e0 = j < nb): nb a multiple of 16, or a divisor
+//          of 16 (then j + (r*nb mod 16) < 16);
+//   writes (ST = Ns, e0 = M*Ns*RAD + k, k < Ns): Ns a multiple of 16, or a
+//          divisor of 16 with Ns*RAD a multiple or a divisor of 16.
+// In both cases (e0 + r*ST) >> 4 = (e0 >> 4) + ((r*ST) >> 4).  With the rows
+// of the I/O functors below and the 32-bit reciprocals of split_line, one B200,
+// before -> after, same bits: 2^20 x 16 ComplexF32 155.6 -> 147.7 us, 27648 x
+// 606 140.8 -> 134.6, 65537 x 16 (Bluestein) 94.1 -> 81.4, 4096 x 4096 2-D
+// 141.3 -> 137.3, rfft 4096 x 16384 128.2 -> 123.1; one-pass complex batches
+// are bound by memory and did not change.
+template <class RL, int RAD, int ST, bool WR> __host__ __device__ constexpr bool const_pad() {
+  return prog_len<RL>() % 2 == 1 || ST % 16 == 0 ||
+         (16 % ST == 0 && (!WR || (ST * RAD) % 16 == 0 || 16 % (ST * RAD) == 0));
+}
+template <class RL, int RAD, int ST, bool WR> struct Slots {
+  int e0, p0;
+  __device__ __forceinline__ explicit Slots(int e) : e0(e), p0(pidx<RL>(e)) {}
+  __device__ __forceinline__ int operator[](int r) const {
+    if constexpr (const_pad<RL, RAD, ST, WR>())
+      return p0 + r * ST + (prog_len<RL>() % 2 == 1 ? 0 : (r * ST) >> 4);
+    else
+      return pidx<RL>(e0 + r * ST);
+  }
+};
+
 // ---------------------------------------------------------------- I/O
 // A stage's input or output is shared memory (SmemIO) or a functor that
 // loads element i of the line / stores element i of the line.
 struct SmemIO {};
 
-// Input functors load element i in two steps: raw(i) issues the memory load,
-// fin(i, v) applies what depends on the element (tables, twiddles).  A stage
-// issues all of its raw loads before any fin, so every data load is in flight
-// before the table loads take registers.
+// An I/O functor hands out one row per butterfly: at<ST>(e0) covers the
+// elements e0 + r*ST of the line.  A row holds the address of e0 and 32-bit
+// element strides, so an access costs one wide multiply-add (or none, where
+// the elements are contiguous) instead of an index product, its widening and
+// the add.  Input rows load element r in two steps: raw(r) issues the memory
+// load, fin(v) applies what depends on the elements (tables, twiddles).  A
+// stage issues all of its raw loads before any fin, so every data load is in
+// flight before the table loads take registers.
 //
 // Cache hints.  A pass reads each input element once, so data loads are
 // streaming (evict-first in L2): the misses of a pass then displace each
@@ -98,104 +131,160 @@ template <typename R> __device__ __forceinline__ void store(cplx<R>* p, cplx<R> 
   else
     *p = v;
 }
+// p + r*step elements: a 32 x 32 -> 64 bit product added to the address.
+template <typename C> __device__ __forceinline__ C* step_ptr(C* p, int step, int r) {
+  return (C*)((uintptr_t)p + (uint64_t)((int64_t)step * (int64_t)(r * (int)sizeof(C))));
+}
+
 template <typename R> struct DirectIn {
   const cplx<R>* __restrict__ g;
   bool ok;
-  __device__ __forceinline__ cplx<R> raw(int i) const {
-    return ok ? __ldcs(g + i) : Sc<R>::mk(R(0), R(0));
+  template <int ST> struct Row {
+    const cplx<R>* __restrict__ p;
+    bool ok;
+    __device__ __forceinline__ cplx<R> raw(int r) const {
+      return ok ? __ldcs(p + r * ST) : Sc<R>::mk(R(0), R(0));
+    }
+    template <int RAD> __device__ __forceinline__ void fin(cplx<R>*) const {}
+  };
+  template <int ST> __device__ __forceinline__ Row<ST> at(int e0) const {
+    return Row<ST>{g + e0, ok};
   }
-  __device__ __forceinline__ cplx<R> fin(int, cplx<R> v) const { return v; }
 };
 template <typename R> struct DirectOut {
   cplx<R>* __restrict__ g;
   bool ok;
   R scale;
   bool cs;
-  __device__ __forceinline__ void operator()(int i, cplx<R> v) const {
-    if (ok) store<R>(g + i, scale == R(1) ? v : cscale<R>(v, scale), cs);
+  template <int ST> struct Row {
+    cplx<R>* __restrict__ p;
+    bool ok;
+    R scale;
+    bool cs;
+    __device__ __forceinline__ void put(int r, cplx<R> v) const {
+      if (ok) store<R>(p + r * ST, scale == R(1) ? v : cscale<R>(v, scale), cs);
+    }
+  };
+  template <int ST> __device__ __forceinline__ Row<ST> at(int e0) const {
+    return Row<ST>{g + e0, ok, scale, cs};
   }
 };
 
-// Element i of a strided line, present when i*ves + voff < vn; the optional
-// table `mul` (the chirp) is indexed by that same value.
+// Elements of a line that are present: i*ves + voff < vn, i.e. i < count.
+__device__ __forceinline__ int present_count(int64_t vn, int ves, int64_t voff, bool ok) {
+  if (!ok || voff >= vn) return 0;
+  if (ves == 0 || vn == INT64_MAX) return INT32_MAX;
+  const int64_t c = (vn - voff + ves - 1) / ves;
+  return c > INT32_MAX ? INT32_MAX : (int)c;
+}
+// Full I/O (Bluestein and root-table passes).  Element i of a strided line,
+// present when i < cnt; the optional table `mul` (the chirp) is read at
+// mul + i*ves (the line's offset included), the twiddle on load
+// (LineArgs::tw_on_load) at tab + i*tab_es.
 template <typename R> struct TileIn {
   const cplx<R>* __restrict__ base;
-  int64_t es;
+  int es, cnt;
   const cplx<R>* __restrict__ mul;
-  int64_t vn, ves, voff;
-  bool ok;
-  const cplx<R>* __restrict__ tab;  // twiddle on load (LineArgs::tw_on_load)
-  int64_t tab_es, tab_off;
-  int tw_dir;
-  __device__ __forceinline__ cplx<R> raw(int i) const {
-    const int64_t vi = (int64_t)i * ves + voff;
-    if (!ok || vi >= vn) return Sc<R>::mk(R(0), R(0));
-    return __ldcs(base + (int64_t)i * es);
-  }
-  __device__ __forceinline__ cplx<R> fin(int i, cplx<R> v) const {
-    const int64_t vi = (int64_t)i * ves + voff;
-    if (!ok || vi >= vn) return v;
-    if (mul) v = cmul<R>(v, __ldg(mul + vi));
-    if (tab) {
-      const cplx<R> w = __ldg(tab + (int64_t)i * tab_es + tab_off);
-      v = tw_dir < 0 ? cmul<R>(v, w) : cmulc<R>(v, w);
+  int ves;
+  const cplx<R>* __restrict__ tab;
+  int tab_es, tw_dir;
+  template <int ST> struct Row {
+    const cplx<R>* p;
+    const cplx<R>* pm;
+    const cplx<R>* pt;
+    int step, mstep, tstep, left, dir;
+    __device__ __forceinline__ cplx<R> raw(int r) const {
+      return r * ST < left ? __ldcs(step_ptr(p, step, r)) : Sc<R>::mk(R(0), R(0));
     }
-    return v;
+    template <int RAD> __device__ __forceinline__ void fin(cplx<R>* v) const {
+      if (pm) {
+#pragma unroll
+        for (int r = 0; r < RAD; ++r)
+          if (r * ST < left) v[r] = cmul<R>(v[r], __ldg(step_ptr(pm, mstep, r)));
+      }
+      if (pt) {
+#pragma unroll
+        for (int r = 0; r < RAD; ++r)
+          if (r * ST < left) {
+            const cplx<R> w = __ldg(step_ptr(pt, tstep, r));
+            v[r] = dir < 0 ? cmul<R>(v[r], w) : cmulc<R>(v[r], w);
+          }
+      }
+    }
+  };
+  template <int ST> __device__ __forceinline__ Row<ST> at(int e0) const {
+    return Row<ST>{base + (int64_t)e0 * es,
+                   mul ? mul + (int64_t)e0 * ves : nullptr,
+                   tab ? tab + (int64_t)e0 * tab_es : nullptr,
+                   es * ST, ves * ST, tab_es * ST, cnt - e0, tw_dir};
   }
 };
-// Store with, in order: the table `mul` (chirp), the twiddle w_N^(dir*l0*i)
-// (hi/lo root tables), the scale.
+
 // prefetch.global.L1: a hint that brings the line into L1 (no register is
 // written; the address is one the kernel reads later).
 __device__ __forceinline__ void prefetch_l1(const void* p) {
   asm volatile("prefetch.global.L1 [%0];" ::"l"(p));
 }
-
+// Store with, in order: the table `mul` (chirp), the twiddle w_N^(dir*l0*i)
+// (full table, or hi/lo root tables), the scale.
 template <typename R> struct TileOut {
   cplx<R>* __restrict__ base;
-  int64_t es;
+  int es, cnt;
   const cplx<R>* __restrict__ mul;
-  int64_t vn, ves, voff;
-  int64_t l0;
+  int ves;
+  uint32_t l0;  // line's twiddle index; l0 * i < 2^31 (tw_N's range)
   const cplx<R>* __restrict__ tw_hi;
   const cplx<R>* __restrict__ tw_lo;
   int tw_shift, tw_dir;
   R scale;
-  bool ok;
   const cplx<R>* __restrict__ tab;  // full twiddle table (precedence over hi/lo)
-  int64_t tab_es, tab_off;
+  int tab_es;
   bool cs;
-  __device__ __forceinline__ void operator()(int i, cplx<R> v) const {
-    const int64_t vi = (int64_t)i * ves + voff;
-    if (!ok || vi >= vn) return;
-    if (mul) v = cmul<R>(v, __ldg(mul + vi));
-    if (tab) {
-      const cplx<R> w = __ldg(tab + (int64_t)i * tab_es + tab_off);
-      v = tw_dir < 0 ? cmul<R>(v, w) : cmulc<R>(v, w);
-    } else if (tw_hi) {
-      const int64_t e = l0 * (int64_t)i;
-      const cplx<R> w = cmul<R>(__ldg(tw_hi + (e >> tw_shift)),
-                                __ldg(tw_lo + (e & ((int64_t(1) << tw_shift) - 1))));
-      v = tw_dir < 0 ? cmul<R>(v, w) : cmulc<R>(v, w);
+  template <int ST> struct Row {
+    cplx<R>* p;
+    const cplx<R>* pm;
+    const cplx<R>* pt;
+    int step, mstep, tstep, left;
+    uint32_t e, estep;
+    const TileOut& o;
+    __device__ __forceinline__ void put(int r, cplx<R> v) const {
+      if (r * ST >= left) return;
+      if (pm) v = cmul<R>(v, __ldg(step_ptr(pm, mstep, r)));
+      if (pt) {
+        const cplx<R> w = __ldg(step_ptr(pt, tstep, r));
+        v = o.tw_dir < 0 ? cmul<R>(v, w) : cmulc<R>(v, w);
+      } else if (o.tw_hi) {
+        const uint32_t x = e + (uint32_t)r * estep;
+        const cplx<R> w = cmul<R>(__ldg(o.tw_hi + (x >> o.tw_shift)),
+                                  __ldg(o.tw_lo + (x & ((1u << o.tw_shift) - 1u))));
+        v = o.tw_dir < 0 ? cmul<R>(v, w) : cmulc<R>(v, w);
+      }
+      if (o.scale != R(1)) v = cscale<R>(v, o.scale);
+      store<R>(step_ptr(p, step, r), v, o.cs);
     }
-    if (scale != R(1)) v = cscale<R>(v, scale);
-    store<R>(base + (int64_t)i * es, v, cs);
-  }
-  // Bring the per-element tables element i's store will read (chirp, full
-  // twiddle table) into L1 ahead of time; the same presence test as above.
-  __device__ __forceinline__ void prefetch(int i) const {
-    const int64_t vi = (int64_t)i * ves + voff;
-    if (!ok || vi >= vn) return;
-    if (mul) prefetch_l1(mul + vi);
-    if (tab) prefetch_l1(tab + (int64_t)i * tab_es + tab_off);
+    // Bring the tables element r's store will read (chirp, full twiddle
+    // table) into L1 ahead of time; the same presence test as above.
+    __device__ __forceinline__ void prefetch(int r) const {
+      if (r * ST >= left) return;
+      if (pm) prefetch_l1(step_ptr(pm, mstep, r));
+      if (pt) prefetch_l1(step_ptr(pt, tstep, r));
+    }
+  };
+  template <int ST> __device__ __forceinline__ Row<ST> at(int e0) const {
+    return Row<ST>{base + (int64_t)e0 * es,
+                   mul ? mul + (int64_t)e0 * ves : nullptr,
+                   tab ? tab + (int64_t)e0 * tab_es : nullptr,
+                   es * ST, ves * ST, tab_es * ST, cnt - e0,
+                   l0 * (uint32_t)e0, l0 * (uint32_t)ST, *this};
   }
 };
 
 // Lean I/O for the common case (LineArgs::plain_io): every element present,
 // no chirp tables, 32-bit strides, twiddle (if any) from a full table.  The
 // line index is clamped to a valid line, so loads need no predicate.
-// `tab` is a generic pointer: the twiddle table in global memory, or the
-// line's slice of it staged in shared memory (then tab_es = 1, tab_off = 0).
+// `tab` is a generic pointer to the line's entries: the twiddle table in
+// global memory, or the line's slice of it staged in shared memory (then
+// tab_es = 1).
 //
 // TW fixes at compile time what a functor multiplies by: kTwRuntime tests
 // `tab` and `tw_dir` at every element; kTwNone has no table; -1 / +1 always
@@ -204,85 +293,97 @@ template <typename R> struct TileOut {
 // take the fixed forms, so their unrolled stages carry no per-element tests
 // of launch-wide values; the arithmetic is the same in every form.
 constexpr int kTwRuntime = 0, kTwNone = 2;
+template <typename R, int TW>
+__device__ __forceinline__ cplx<R> tw_mul(cplx<R> v, cplx<R> w, int tw_dir) {
+  if constexpr (TW == -1)
+    return cmul<R>(v, w);
+  else if constexpr (TW == 1)
+    return cmulc<R>(v, w);
+  else
+    return tw_dir < 0 ? cmul<R>(v, w) : cmulc<R>(v, w);
+}
 template <typename R, int TW = kTwRuntime> struct PlainIn {
   const cplx<R>* __restrict__ base;
   int es;
   const cplx<R>* tab;  // twiddle on load (LineArgs::tw_on_load)
-  int tab_es, tab_off, tw_dir;
-  __device__ __forceinline__ bool has_tab() const {
-    return TW == kTwRuntime ? tab != nullptr : TW != kTwNone;
-  }
-  __device__ __forceinline__ cplx<R> twm(cplx<R> v, cplx<R> w) const {
-    if constexpr (TW == -1)
-      return cmul<R>(v, w);
-    else if constexpr (TW == 1)
-      return cmulc<R>(v, w);
-    else
-      return tw_dir < 0 ? cmul<R>(v, w) : cmulc<R>(v, w);
-  }
-  __device__ __forceinline__ cplx<R> raw(int i) const { return __ldcs(base + (int64_t)(i * es)); }
-  __device__ __forceinline__ cplx<R> fin(int i, cplx<R> v) const {
-    if (has_tab()) v = twm(v, tab[i * tab_es + tab_off]);
-    return v;
-  }
-  // The twiddles of butterfly j's inputs i = j + r*nb (tw_elem's product):
-  // ceil(RAD/4) entries of its own plus the line's steps t(c*nb), c = 1..3.
-  template <int RAD>
-  __device__ __forceinline__ void fin_bfly(int j, int nb, cplx<R>* v) const {
-    if (!has_tab()) return;
-    if constexpr (RAD < 4) {
+  int tab_es, tw_dir;
+  template <int ST> struct Row {
+    const cplx<R>* p;
+    int step;
+    const cplx<R>* pt;  // twiddle of element e0
+    const cplx<R>* t0;  // the line's entry 0
+    int tstep, dir;
+    __device__ __forceinline__ cplx<R> raw(int r) const { return __ldcs(step_ptr(p, step, r)); }
+    // The twiddles of the elements j + r*ST, ST = nb (tw_elem's product):
+    // ceil(RAD/4) entries of its own plus the line's steps t(c*nb), c = 1..3.
+    template <int RAD> __device__ __forceinline__ void fin(cplx<R>* v) const {
+      if (!(TW == kTwRuntime ? t0 != nullptr : TW != kTwNone)) return;
+      if constexpr (RAD < 4) {
 #pragma unroll
-      for (int r = 0; r < RAD; ++r) v[r] = fin(j + r * nb, v[r]);
-    } else {
-      cplx<R> s[4];
+        for (int r = 0; r < RAD; ++r) v[r] = tw_mul<R, TW>(v[r], *step_ptr(pt, tstep, r), dir);
+      } else {
+        cplx<R> s[4];
 #pragma unroll
-      for (int c = 1; c < 4; ++c) s[c] = tab[c * nb * tab_es + tab_off];
+        for (int c = 1; c < 4; ++c) s[c] = *step_ptr(t0, tstep, c);
 #pragma unroll
-      for (int a = 0; a < RAD; a += 4) {
-        const cplx<R> b = tab[(j + a * nb) * tab_es + tab_off];
+        for (int a = 0; a < RAD; a += 4) {
+          const cplx<R> b = *step_ptr(pt, tstep, a);
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          if (a + c < RAD) {
-            const cplx<R> w = c == 0 ? b : cmul<R>(b, s[c]);
-            v[a + c] = twm(v[a + c], w);
+          for (int c = 0; c < 4; ++c) {
+            if (a + c < RAD) {
+              const cplx<R> w = c == 0 ? b : cmul<R>(b, s[c]);
+              v[a + c] = tw_mul<R, TW>(v[a + c], w, dir);
+            }
           }
         }
       }
     }
+  };
+  template <int ST> __device__ __forceinline__ Row<ST> at(int e0) const {
+    return Row<ST>{base + (int64_t)e0 * es, es * ST, tab + (int64_t)e0 * tab_es, tab, tab_es * ST,
+                   tw_dir};
   }
 };
-template <class In> struct InHasBfly : std::false_type {};
-template <typename R, int TW> struct InHasBfly<PlainIn<R, TW>> : std::true_type {};
 template <typename R, int TW = kTwRuntime, bool SCALE = true> struct PlainOut {
   cplx<R>* __restrict__ base;
   int es;
   const cplx<R>* tab;
-  int tab_es, tab_off, tw_dir;
+  int tab_es, tw_dir;
   R scale;
   bool ok;
   bool cs;
-  __device__ __forceinline__ void operator()(int i, cplx<R> v) const {
-    if (TW == kTwRuntime ? tab != nullptr : TW != kTwNone) {
-      const cplx<R> w = tab[i * tab_es + tab_off];
-      if constexpr (TW == -1)
-        v = cmul<R>(v, w);
-      else if constexpr (TW == 1)
-        v = cmulc<R>(v, w);
-      else
-        v = tw_dir < 0 ? cmul<R>(v, w) : cmulc<R>(v, w);
+  template <int ST> struct Row {
+    cplx<R>* p;
+    int step;
+    const cplx<R>* pt;
+    const cplx<R>* t0;
+    int tstep, dir;
+    R scale;
+    bool ok, cs;
+    __device__ __forceinline__ void put(int r, cplx<R> v) const {
+      if (TW == kTwRuntime ? t0 != nullptr : TW != kTwNone)
+        v = tw_mul<R, TW>(v, *step_ptr(pt, tstep, r), dir);
+      if (SCALE && scale != R(1)) v = cscale<R>(v, scale);
+      if (ok) store<R>(step_ptr(p, step, r), v, cs);
     }
-    if (SCALE && scale != R(1)) v = cscale<R>(v, scale);
-    if (ok) store<R>(base + (int64_t)(i * es), v, cs);
+  };
+  template <int ST> __device__ __forceinline__ Row<ST> at(int e0) const {
+    return Row<ST>{base + (int64_t)e0 * es, es * ST, tab + (int64_t)e0 * tab_es, tab, tab_es * ST,
+                   tw_dir, scale, ok, cs};
   }
 };
 
-// Element i of a line held flat (unpadded) in shared memory: the landing
-// buffer of a bulk copy (fast_stream_kernel).  Stage 0 then overwrites the
-// same buffer in the padded layout, after a barrier.
+// A line held flat (unpadded) in shared memory: the landing buffer of a bulk
+// copy (fast_stream_kernel).  Stage 0 then overwrites the same buffer in the
+// padded layout, after a barrier.
 template <typename R> struct FlatIn {
   const cplx<R>* p;
-  __device__ __forceinline__ cplx<R> raw(int i) const { return p[i]; }
-  __device__ __forceinline__ cplx<R> fin(int, cplx<R> v) const { return v; }
+  template <int ST> struct Row {
+    const cplx<R>* p;
+    __device__ __forceinline__ cplx<R> raw(int r) const { return p[r * ST]; }
+    template <int RAD> __device__ __forceinline__ void fin(cplx<R>*) const {}
+  };
+  template <int ST> __device__ __forceinline__ Row<ST> at(int e0) const { return Row<ST>{p + e0}; }
 };
 template <class In> struct InIsSmem : std::false_type {};
 template <typename R> struct InIsSmem<FlatIn<R>> : std::true_type {};
@@ -312,12 +413,14 @@ __device__ __forceinline__ void fast_stage(cplx<R>* buf, const In& in, const Out
   for (int q = 0; q < UM; ++q) {
     const int j = u + q * T;
     if (nb % T == 0 || j < nb) {
+      if constexpr (GIN) {
+        const auto row = in.template at<nb>(j);
 #pragma unroll
-      for (int r = 0; r < RAD; ++r) {
-        if constexpr (GIN)
-          v[q][r] = in.raw(j + r * nb);
-        else
-          v[q][r] = buf[pidx<RL>(j + r * nb)];
+        for (int r = 0; r < RAD; ++r) v[q][r] = row.raw(r);
+      } else {
+        const Slots<RL, RAD, nb, false> sl(j);
+#pragma unroll
+        for (int r = 0; r < RAD; ++r) v[q][r] = buf[sl[r]];
       }
     }
   }
@@ -325,14 +428,7 @@ __device__ __forceinline__ void fast_stage(cplx<R>* buf, const In& in, const Out
 #pragma unroll
     for (int q = 0; q < UM; ++q) {
       const int j = u + q * T;
-      if (nb % T == 0 || j < nb) {
-        if constexpr (InHasBfly<In>::value) {
-          in.template fin_bfly<RAD>(j, nb, v[q]);
-        } else {
-#pragma unroll
-          for (int r = 0; r < RAD; ++r) v[q][r] = in.fin(j + r * nb, v[q][r]);
-        }
-      }
+      if (nb % T == 0 || j < nb) in.template at<nb>(j).template fin<RAD>(v[q]);
     }
   }
   // in place: all reads of the line finish before any write, unless one side
@@ -342,7 +438,8 @@ __device__ __forceinline__ void fast_stage(cplx<R>* buf, const In& in, const Out
   for (int q = 0; q < UM; ++q) {
     const int j = u + q * T;
     if (nb % T == 0 || j < nb) {
-      const int k = (Ns == 1) ? 0 : j % Ns;
+      // k = j mod Ns (the last stage has Ns = nb > j)
+      const int k = Ns == 1 ? 0 : (Ns == nb ? j : (int)((unsigned)j % (unsigned)Ns));
       if constexpr (Ns > 1) {
         const cplx<R>* w = tw + tw_offset<RL, S>() + k;  // entry (r-1)*Ns + k
 #pragma unroll
@@ -353,12 +450,14 @@ __device__ __forceinline__ void fast_stage(cplx<R>* buf, const In& in, const Out
       else
         butterfly<R, RAD, DIR>(v[q], pcs);
       const int base = (j - k) * RAD + k;
+      if constexpr (GOUT) {
+        const auto row = out.template at<Ns>(base);
 #pragma unroll
-      for (int r = 0; r < RAD; ++r) {
-        if constexpr (GOUT)
-          out(base + r * Ns, v[q][r]);
-        else
-          buf[pidx<RL>(base + r * Ns)] = v[q][r];
+        for (int r = 0; r < RAD; ++r) row.put(r, v[q][r]);
+      } else {
+        const Slots<RL, RAD, Ns, true> sl(base);
+#pragma unroll
+        for (int r = 0; r < RAD; ++r) buf[sl[r]] = v[q][r];
       }
     }
   }
@@ -381,7 +480,7 @@ __device__ __forceinline__ void fast_prog(cplx<R>* buf, const In& in, const Out&
 // otherwise wait out the memory latency with nothing else to run.
 template <typename R, class RL, int T>
 __device__ __forceinline__ void prefetch_store_tables(const TileOut<R>& o, int u) {
-  if (!o.ok || !(o.mul || o.tab)) return;
+  if (!(o.mul || o.tab)) return;
   constexpr int S = RL::n - 1;
   constexpr int RAD = RL::r[S];
   constexpr int Ns = ns_before<RL, S>();
@@ -391,10 +490,10 @@ __device__ __forceinline__ void prefetch_store_tables(const TileOut<R>& o, int u
   for (int q = 0; q < UM; ++q) {
     const int j = u + q * T;
     if (nb % T == 0 || j < nb) {
-      const int k = (Ns == 1) ? 0 : j % Ns;
-      const int base = (j - k) * RAD + k;
+      // the last stage's Ns = nb > j, so its outputs are j + r*Ns
+      const auto row = o.template at<Ns>(j);
 #pragma unroll
-      for (int r = 0; r < RAD; ++r) o.prefetch(base + r * Ns);
+      for (int r = 0; r < RAD; ++r) row.prefetch(r);
     }
   }
 }
@@ -562,6 +661,24 @@ template <typename R, class RL, int T, bool MID, bool PLAIN> struct TileBounds {
                  ? 2
                  : 1);
 };
+// Batch levels of line l (LineIO): l = q0 + m0*(q1 + m1*q2).  Launches of
+// fewer than 2^31 lines divide by 32-bit reciprocals made on the host
+// (LineArgs::d0, d1); the 64-bit divisions they replace took about a
+// thousand cycles before a block could issue its first load.
+__device__ __forceinline__ void split_line(const LineArgs& a, int64_t l, int64_t* q0, int64_t* q1,
+                                           int64_t* q2) {
+  if (a.d0.mul) {
+    const uint32_t x = (uint32_t)l, t = a.d0.quot(x), w = a.d1.quot(t);
+    *q0 = x - t * (uint32_t)a.m0;
+    *q1 = t - w * (uint32_t)a.m1;
+    *q2 = w;
+  } else {
+    const int64_t t = l / a.m0;
+    *q0 = l % a.m0;
+    *q1 = t % a.m1;
+    *q2 = t / a.m1;
+  }
+}
 // Whether a tile launch reserves shared memory for a staged twiddle slice:
 // only four-step passes whose slice follows the second batch level.
 __host__ __device__ inline bool stages_twiddles(const LineArgs& a, int L) {
@@ -606,23 +723,27 @@ __global__ void __launch_bounds__(TileThreads<R, T, MID>::value,
   const int g = threadIdx.x, u = threadIdx.y;
   const int G = a.G, P = tile_pitch(LPAD, G, (int)sizeof(C));
   C* buf = (C*)smraw + g * P;
-  // one thread per line splits its index into the batch levels (64-bit
-  // divisions) and leaves the results in shared memory for the others
-  // (four arrays of G entries, so a warp's reads are consecutive)
+  // one thread per line splits its index into the batch levels and leaves the
+  // results in shared memory for the others (four arrays of G entries, so a
+  // warp's reads are consecutive); lb[g] holds the elements present on load
+  // and on store where a window limits them
   int64_t* lb = (int64_t*)((C*)smraw + (size_t)G * P);
   const int64_t line = (int64_t)blockIdx.x * G + g;
   const bool ok = line < a.nlines;
   if (u == 0) {
-    const int64_t l = ok ? line : 0;
-    const int64_t q0 = l % a.m0, t = l / a.m0;
-    const int64_t q1 = t % a.m1, q2 = t / a.m1;
-    lb[g] = q0;
+    int64_t q0, q1, q2;
+    split_line(a, ok ? line : 0, &q0, &q1, &q2);
     lb[G + g] = q0 * a.ld.s0 + q1 * a.ld.s1 + q2 * a.ld.s2;
     lb[2 * G + g] = q0 * a.st.s0 + q1 * a.st.s1 + q2 * a.st.s2;
-    lb[3 * G + g] = a.tw_level ? q1 : q0;
+    if constexpr (PLAIN && !MID) {
+      lb[3 * G + g] = a.tw_level ? q1 : q0;
+    } else {
+      lb[g] = (int64_t)present_count(a.ld.vn, (int)a.ld.ves, q0 * a.ld.vls, ok) |
+              (int64_t)present_count(a.st.vn, (int)a.st.ves, q0 * a.st.vls, ok) << 32;
+      lb[3 * G + g] = q0 | (a.tw_level ? q1 : q0) << 32;  // both below 2^31 (use_tile)
+    }
   }
   __syncthreads();
-  const int64_t l0 = lb[g], lt = lb[3 * G + g];
   const C* tw = (const C*)a.prog.tw;
   const R* pcs = (const R*)a.prime_cs;
   const C* ib = (const C*)a.in + lb[G + g];
@@ -631,9 +752,10 @@ __global__ void __launch_bounds__(TileThreads<R, T, MID>::value,
     const C* tin = a.tw_on_load ? (const C*)a.tw_tab : nullptr;
     const C* tout = a.tw_on_load ? nullptr : (const C*)a.tw_tab;
     const C* st = stage_twiddles<C>(a, lb + 3 * G, G, L, (C*)(lb + 4 * G), g + G * u, G * T);
-    const int tes = st ? 1 : (int)a.tw_es, toff = st ? 0 : (int)(lt * a.tw_ls);
-    const C* ti = tin ? (st ? st : tin) : nullptr;
-    const C* to = tout ? (st ? st : tout) : nullptr;
+    const int tes = st ? 1 : (int)a.tw_es;
+    const int64_t toff = lb[3 * G + g] * a.tw_ls;
+    const C* ti = tin ? (st ? st : tin + toff) : nullptr;
+    const C* to = tout ? (st ? st : tout + toff) : nullptr;
     const int ies = (int)a.ld.es, oes = (int)a.st.es;
     const bool cs = a.st_stream != 0;
     // The lean passes of the four-step and 2-D schedules -- no twiddle, or a
@@ -642,29 +764,29 @@ __global__ void __launch_bounds__(TileThreads<R, T, MID>::value,
     // lean launch takes the run-time form.
     const bool fixed = (R)a.scale == R(1) && !(ti && to) && (!(ti || to) || a.tw_dir == a.dir1);
     if (fixed && !ti && !to) {
-      const PlainIn<R, kTwNone> in{ib, ies, nullptr, 0, 0, 0};
-      const PlainOut<R, kTwNone, false> out{ob, oes, nullptr, 0, 0, 0, R(1), ok, cs};
+      const PlainIn<R, kTwNone> in{ib, ies, nullptr, 0, 0};
+      const PlainOut<R, kTwNone, false> out{ob, oes, nullptr, 0, 0, R(1), ok, cs};
       if (a.dir1 < 0)
         fast_prog<R, -1, RL, T>(buf, in, out, tw, pcs, u);
       else
         fast_prog<R, 1, RL, T>(buf, in, out, tw, pcs, u);
     } else if (fixed && ti) {
-      const PlainOut<R, kTwNone, false> out{ob, oes, nullptr, 0, 0, 0, R(1), ok, cs};
+      const PlainOut<R, kTwNone, false> out{ob, oes, nullptr, 0, 0, R(1), ok, cs};
       if (a.dir1 < 0)
-        fast_prog<R, -1, RL, T>(buf, PlainIn<R, -1>{ib, ies, ti, tes, toff, -1}, out, tw, pcs, u);
+        fast_prog<R, -1, RL, T>(buf, PlainIn<R, -1>{ib, ies, ti, tes, -1}, out, tw, pcs, u);
       else
-        fast_prog<R, 1, RL, T>(buf, PlainIn<R, 1>{ib, ies, ti, tes, toff, 1}, out, tw, pcs, u);
+        fast_prog<R, 1, RL, T>(buf, PlainIn<R, 1>{ib, ies, ti, tes, 1}, out, tw, pcs, u);
     } else if (fixed) {
-      const PlainIn<R, kTwNone> in{ib, ies, nullptr, 0, 0, 0};
+      const PlainIn<R, kTwNone> in{ib, ies, nullptr, 0, 0};
       if (a.dir1 < 0)
-        fast_prog<R, -1, RL, T>(buf, in, PlainOut<R, -1, false>{ob, oes, to, tes, toff, -1, R(1), ok, cs},
+        fast_prog<R, -1, RL, T>(buf, in, PlainOut<R, -1, false>{ob, oes, to, tes, -1, R(1), ok, cs},
                                 tw, pcs, u);
       else
-        fast_prog<R, 1, RL, T>(buf, in, PlainOut<R, 1, false>{ob, oes, to, tes, toff, 1, R(1), ok, cs},
+        fast_prog<R, 1, RL, T>(buf, in, PlainOut<R, 1, false>{ob, oes, to, tes, 1, R(1), ok, cs},
                                tw, pcs, u);
     } else {
-      const PlainIn<R> in{ib, ies, ti, tes, toff, a.tw_dir};
-      const PlainOut<R> out{ob, oes, to, tes, toff, a.tw_dir, (R)a.scale, ok, cs};
+      const PlainIn<R> in{ib, ies, ti, tes, a.tw_dir};
+      const PlainOut<R> out{ob, oes, to, tes, a.tw_dir, (R)a.scale, ok, cs};
       if (a.dir1 < 0)
         fast_prog<R, -1, RL, T>(buf, in, out, tw, pcs, u);
       else
@@ -673,12 +795,16 @@ __global__ void __launch_bounds__(TileThreads<R, T, MID>::value,
   } else {
     const C* tin = a.tw_on_load ? (const C*)a.tw_tab : nullptr;
     const C* tout = a.tw_on_load ? nullptr : (const C*)a.tw_tab;
-    const TileIn<R> in{ib, a.ld.es, (const C*)a.ld.mul, a.ld.vn, a.ld.ves, l0 * a.ld.vls, ok,
-                       tin, a.tw_es, lt * a.tw_ls, a.tw_dir};
-    const TileOut<R> out{ob, a.st.es, (const C*)a.st.mul, a.st.vn, a.st.ves, l0 * a.st.vls, lt,
-                         a.tw_N ? (const C*)a.tw_hi : nullptr, (const C*)a.tw_lo, a.tw_shift,
-                         a.tw_dir, (R)a.scale, ok, tout, a.tw_es, lt * a.tw_ls,
-                         a.st_stream != 0};
+    const int cin = (int)lb[g], cout = (int)(lb[g] >> 32);
+    const int64_t l0 = (uint32_t)lb[3 * G + g], lt = lb[3 * G + g] >> 32;
+    const TileIn<R> in{ib, (int)a.ld.es, cin,
+                       a.ld.mul ? (const C*)a.ld.mul + l0 * a.ld.vls : nullptr, (int)a.ld.ves,
+                       tin ? tin + lt * a.tw_ls : nullptr, (int)a.tw_es, a.tw_dir};
+    const TileOut<R> out{ob, (int)a.st.es, cout,
+                         a.st.mul ? (const C*)a.st.mul + l0 * a.st.vls : nullptr, (int)a.st.ves,
+                         (uint32_t)lt, a.tw_N ? (const C*)a.tw_hi : nullptr, (const C*)a.tw_lo,
+                         a.tw_shift, a.tw_dir, (R)a.scale,
+                         tout ? tout + lt * a.tw_ls : nullptr, (int)a.tw_es, a.st_stream != 0};
     prefetch_store_tables<R, RL, T>(out, u);
     if constexpr (MID) {
       const C* __restrict__ mid = (const C*)a.mid;
@@ -812,9 +938,13 @@ __device__ __forceinline__ void tma_load_4d(void* dst, const void* tmap, int x, 
 // Element i of line g read from a landed tile (this thread's line: t + g,
 // stride G); the four-step twiddle on the loads as PlainIn applies it.
 template <typename R> struct TmaIn : PlainIn<R> {
-  __device__ __forceinline__ cplx<R> raw(int i) const { return this->base[i * this->es]; }
+  template <int ST> struct Row : PlainIn<R>::template Row<ST> {
+    __device__ __forceinline__ cplx<R> raw(int r) const { return this->p[r * this->step]; }
+  };
+  template <int ST> __device__ __forceinline__ Row<ST> at(int e0) const {
+    return Row<ST>{PlainIn<R>::template at<ST>(e0)};
+  }
 };
-template <typename R> struct InHasBfly<TmaIn<R>> : std::true_type {};
 template <typename R> struct InIsSmem<TmaIn<R>> : std::true_type {};
 
 template <typename R, class RL, int T>
@@ -839,9 +969,8 @@ __global__ void __launch_bounds__(TileThreads<R, T, false>::value,
   const uint32_t box_bytes = (uint32_t)(q.boxr * G * (int)sizeof(C));
   // the copies of this block's k-th tile into buffer b (thread 0 only)
   auto issue = [&](int64_t k, int b) {
-    const int64_t line = (first + k * step) * G;
-    const int64_t q0 = line % a.m0, t = line / a.m0;
-    const int64_t q1 = t % a.m1, q2 = t / a.m1;
+    int64_t q0, q1, q2;
+    split_line(a, (first + k * step) * G, &q0, &q1, &q2);
     unsigned char* dst = smraw + (size_t)b * q.buf_bytes;
     mbar_expect_tx(bar + b, tile_bytes);
     for (int r = 0; r < q.nbox; ++r)
@@ -869,20 +998,19 @@ __global__ void __launch_bounds__(TileThreads<R, T, false>::value,
     if (!__syncthreads_and(got)) break;
     const int64_t nx = k + q.nbuf - 1;
     if (tid == 0 && nx < nmine) issue(nx, (int)(nx % q.nbuf));
-    const int64_t line = (first + k * step) * G + g;
-    const int64_t q0 = line % a.m0, t = line / a.m0;
-    const int64_t q1 = t % a.m1, q2 = t / a.m1;
+    int64_t q0, q1, q2;
+    split_line(a, (first + k * step) * G + g, &q0, &q1, &q2);
     const int64_t lt = a.tw_level ? q1 : q0;
     C* tile = (C*)(smraw + (size_t)b * q.buf_bytes);
     TmaIn<R> in;
     in.base = tile + g;
     in.es = G;
-    in.tab = tin;
+    in.tab = tin ? tin + lt * a.tw_ls : nullptr;
     in.tab_es = (int)a.tw_es;
-    in.tab_off = (int)(lt * a.tw_ls);
     in.tw_dir = a.tw_dir;
     const PlainOut<R> out{(C*)a.out + q0 * a.st.s0 + q1 * a.st.s1 + q2 * a.st.s2, (int)a.st.es,
-                          tout, (int)a.tw_es, (int)(lt * a.tw_ls), a.tw_dir, (R)a.scale, true,
+                          tout ? tout + lt * a.tw_ls : nullptr, (int)a.tw_es, a.tw_dir,
+                          (R)a.scale, true,
                           a.st_stream != 0};
     if (a.dir1 < 0)
       fast_prog<R, -1, RL, T>(tile + g * P, in, out, tw, pcs, u);
@@ -965,9 +1093,8 @@ __global__ void __launch_bounds__(512, 2) fast_tc_tile_kernel(const LineArgs a) 
   const int64_t line = (int64_t)blockIdx.x * G + g;
   const bool ok = line < a.nlines;
   if (u == 0) {
-    const int64_t l = ok ? line : 0;
-    const int64_t q0 = l % a.m0, t = l / a.m0;
-    const int64_t q1 = t % a.m1, q2 = t / a.m1;
+    int64_t q0, q1, q2;
+    split_line(a, ok ? line : 0, &q0, &q1, &q2);
     lb[G + g] = q0 * a.ld.s0 + q1 * a.ld.s1 + q2 * a.ld.s2;
     lb[2 * G + g] = q0 * a.st.s0 + q1 * a.st.s1 + q2 * a.st.s2;
     lb[3 * G + g] = a.tw_level ? q1 : q0;
@@ -981,11 +1108,11 @@ __global__ void __launch_bounds__(512, 2) fast_tc_tile_kernel(const LineArgs a) 
   const C* tout = a.tw_on_load ? nullptr : (const C*)a.tw_tab;
   const C* st = stage_twiddles<C>(a, lb + 3 * G, G, prog_len<RL>(), (C*)(slot + 2), g + G * u,
                                   G * T);
-  const int tes = st ? 1 : (int)a.tw_es, toff = st ? 0 : (int)(lt * a.tw_ls);
+  const int tes = st ? 1 : (int)a.tw_es;
   const PlainIn<float> in{(const C*)a.in + lb[G + g], (int)a.ld.es,
-                          tin ? (st ? st : tin) : nullptr, tes, toff, a.tw_dir};
+                          tin ? (st ? st : tin + lt * a.tw_ls) : nullptr, tes, a.tw_dir};
   const PlainOut<float> out{(C*)a.out + lb[2 * G + g], (int)a.st.es,
-                            tout ? (st ? st : tout) : nullptr, tes, toff, a.tw_dir,
+                            tout ? (st ? st : tout + lt * a.tw_ls) : nullptr, tes, a.tw_dir,
                             (float)a.scale, ok, a.st_stream != 0};
   const C* tw = (const C*)a.prog.tw;
   const float* pcs = (const float*)a.prime_cs;
@@ -1019,6 +1146,18 @@ template <typename K> static cudaError_t configure(K k, size_t smem, int* set) {
   e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e == cudaSuccess && dev < 64) set[dev] = (int)smem;
   return e;
+}
+
+// The launch's arguments with the reciprocals split_line divides by.
+static LineArgs with_divisors(LineArgs a) {
+  const int64_t lim = int64_t(1) << 31;
+  if (a.nlines < lim && a.m0 < lim && a.m1 < lim) {
+    a.d0 = Divisor((uint32_t)a.m0);
+    a.d1 = Divisor((uint32_t)a.m1);
+  } else {
+    a.d0 = a.d1 = Divisor();
+  }
+  return a;
 }
 
 // Describe a failed launch: the launch shape and the kernel's attributes.
@@ -1151,7 +1290,8 @@ template <typename R, class RL, int T> struct FastEntry {
       if (q.ntiles <= 0) return cudaSuccess;
       const int64_t cap = (int64_t)per_sm * nsm;
       const int64_t nblk = q.ntiles < cap ? q.ntiles : cap;
-      k<<<dim3((unsigned)nblk), dim3(a.G, T), smem, s>>>(a, *(const CUtensorMap*)tmap, q);
+      k<<<dim3((unsigned)nblk), dim3(a.G, T), smem, s>>>(with_divisors(a),
+                                                         *(const CUtensorMap*)tmap, q);
       e = cudaGetLastError();
       if (e != cudaSuccess) launch_failure(k, "tensor-copy tile launch", L, T, a.G, smem, e);
       return e;
@@ -1202,7 +1342,7 @@ template <typename R, class RL, int T> struct FastEntry {
       }
       const int64_t nblk = (a.nlines + a.G - 1) / a.G;
       if (nblk <= 0) return cudaSuccess;
-      k<<<dim3((unsigned)nblk), dim3(a.G, T), smem, s>>>(a);
+      k<<<dim3((unsigned)nblk), dim3(a.G, T), smem, s>>>(with_divisors(a));
       e = cudaGetLastError();
       if (e != cudaSuccess) launch_failure(k, "tensor-core tile launch", L, T, a.G, smem, e);
       return e;
@@ -1230,7 +1370,7 @@ template <typename R, class RL, int T> struct FastEntry {
     }
     const int64_t nblk = (a.nlines + a.G - 1) / a.G;
     if (nblk <= 0) return cudaSuccess;
-    k<<<dim3((unsigned)nblk), dim3(a.G, T), smem, s>>>(a);
+    k<<<dim3((unsigned)nblk), dim3(a.G, T), smem, s>>>(with_divisors(a));
     e = cudaGetLastError();
     if (e != cudaSuccess) launch_failure(k, "tile launch", L, T, a.G, smem, e);
     return e;

@@ -38,6 +38,24 @@ struct StageProg {
   const void* tw;
 };
 
+// Division of 32-bit values below 2^31 by a divisor d >= 1 known on the host:
+// with 2^s >= d > 2^(s-1) and mul = ceil(2^(31+s) / d), x/d = (x*mul) >> (31+s)
+// for every x < 2^31, as x * (mul*d - 2^(31+s)) < 2^31 * d <= 2^(31+s).
+struct Divisor {
+  uint32_t mul, shift;
+  Divisor() = default;
+  explicit Divisor(uint32_t d) {
+    uint32_t s = 0;
+    while ((uint64_t(1) << s) < d) ++s;
+    shift = 31 + s;
+    mul = (uint32_t)(((uint64_t(1) << shift) + d - 1) / d);
+  }
+#ifdef __CUDACC__
+  __host__ __device__ __forceinline__
+#endif
+  uint32_t quot(uint32_t x) const { return (uint32_t)(((uint64_t)x * mul) >> shift); }
+};
+
 struct LineArgs {
   const void* in;
   void* out;
@@ -74,6 +92,8 @@ struct LineArgs {
                         // specialised kernels store it evict-first
   uint64_t wait_ns;     // limit of a wait on the block's own asynchronous
                         // work (tensor-core products); 0: kWaitNsDefault
+  Divisor d0, d1;       // m0 and m1 (set by the tile launches; mul 0: divide
+                        // in 64 bits)
 };
 
 // Shared-memory pitch (elements) of the lines of a tile block.  A warp holds

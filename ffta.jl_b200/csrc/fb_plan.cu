@@ -649,9 +649,10 @@ static void use_tile(const fb_plan_s* P, Pass& p, const std::vector<int>& radice
   // needed and every 32-bit offset fits.  Set for generic passes too: a
   // four-step twiddle on the loads of a lean pass is tw_elem's product in
   // both kernels, so they keep equal bits.
+  bool small;
   {
     const int64_t L = p.a.prog.L;
-    const bool small = std::llabs(p.a.ld.es) * L < (int64_t(1) << 31) &&
+    small = std::llabs(p.a.ld.es) * L < (int64_t(1) << 31) &&
                        std::llabs(p.a.st.es) * L < (int64_t(1) << 31) &&
                        (!p.a.tw_tab || (L * p.a.tw_es + p.a.tw_ls * (int64_t)p.a.nlines) < (int64_t(1) << 31));
     p.a.plain_io = !p.a.mid && !p.a.ld.mul && !p.a.st.mul && p.a.ld.vn == INT64_MAX &&
@@ -659,6 +660,8 @@ static void use_tile(const fb_plan_s* P, Pass& p, const std::vector<int>& radice
                    p.a.ld.count == L && p.a.st.count == L;
   }
   if (P->flags & 1) return;
+  // the tile kernels address a line's elements and windows with 32 bits
+  if (!small || (!p.a.plain_io && p.a.nlines >= (int64_t(1) << 31))) return;
   const FastFn* ff = find_fast(P->dtype, p.a.prog.L, radices);
   if (!ff || (int)ff->lpad != p.a.Lpad) return;
   if (p.a.mid && (p.a.dir1 > 0 || p.a.dir2 < 0)) return;
