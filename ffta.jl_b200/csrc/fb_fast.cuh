@@ -170,13 +170,6 @@ template <typename R> struct DirectOut {
   }
 };
 
-// Elements of a line that are present: i*ves + voff < vn, i.e. i < count.
-__device__ __forceinline__ int present_count(int64_t vn, int ves, int64_t voff, bool ok) {
-  if (!ok || voff >= vn) return 0;
-  if (ves == 0 || vn == INT64_MAX) return INT32_MAX;
-  const int64_t c = (vn - voff + ves - 1) / ves;
-  return c > INT32_MAX ? INT32_MAX : (int)c;
-}
 // Full I/O (Bluestein and root-table passes).  Element i of a strided line,
 // present when i < cnt; the optional table `mul` (the chirp) is read at
 // mul + i*ves (the line's offset included), the twiddle on load
@@ -661,24 +654,6 @@ template <typename R, class RL, int T, bool MID, bool PLAIN> struct TileBounds {
                  ? 2
                  : 1);
 };
-// Batch levels of line l (LineIO): l = q0 + m0*(q1 + m1*q2).  Launches of
-// fewer than 2^31 lines divide by 32-bit reciprocals made on the host
-// (LineArgs::d0, d1); the 64-bit divisions they replace took about a
-// thousand cycles before a block could issue its first load.
-__device__ __forceinline__ void split_line(const LineArgs& a, int64_t l, int64_t* q0, int64_t* q1,
-                                           int64_t* q2) {
-  if (a.d0.mul) {
-    const uint32_t x = (uint32_t)l, t = a.d0.quot(x), w = a.d1.quot(t);
-    *q0 = x - t * (uint32_t)a.m0;
-    *q1 = t - w * (uint32_t)a.m1;
-    *q2 = w;
-  } else {
-    const int64_t t = l / a.m0;
-    *q0 = l % a.m0;
-    *q1 = t % a.m1;
-    *q2 = t / a.m1;
-  }
-}
 // Whether a tile launch reserves shared memory for a staged twiddle slice:
 // only four-step passes whose slice follows the second batch level.
 __host__ __device__ inline bool stages_twiddles(const LineArgs& a, int L) {
@@ -738,8 +713,8 @@ __global__ void __launch_bounds__(TileThreads<R, T, MID>::value,
     if constexpr (PLAIN && !MID) {
       lb[3 * G + g] = a.tw_level ? q1 : q0;
     } else {
-      lb[g] = (int64_t)present_count(a.ld.vn, (int)a.ld.ves, q0 * a.ld.vls, ok) |
-              (int64_t)present_count(a.st.vn, (int)a.st.ves, q0 * a.st.vls, ok) << 32;
+      lb[g] = (int64_t)present_count(a.ld.vn, a.ld.ves, q0 * a.ld.vls, ok) |
+              (int64_t)present_count(a.st.vn, a.st.ves, q0 * a.st.vls, ok) << 32;
       lb[3 * G + g] = q0 | (a.tw_level ? q1 : q0) << 32;  // both below 2^31 (use_tile)
     }
   }
@@ -1146,18 +1121,6 @@ template <typename K> static cudaError_t configure(K k, size_t smem, int* set) {
   e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e == cudaSuccess && dev < 64) set[dev] = (int)smem;
   return e;
-}
-
-// The launch's arguments with the reciprocals split_line divides by.
-static LineArgs with_divisors(LineArgs a) {
-  const int64_t lim = int64_t(1) << 31;
-  if (a.nlines < lim && a.m0 < lim && a.m1 < lim) {
-    a.d0 = Divisor((uint32_t)a.m0);
-    a.d1 = Divisor((uint32_t)a.m1);
-  } else {
-    a.d0 = a.d1 = Divisor();
-  }
-  return a;
 }
 
 // Describe a failed launch: the launch shape and the kernel's attributes.

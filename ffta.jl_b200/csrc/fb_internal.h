@@ -27,17 +27,6 @@ struct LineIO {
   int count;        // elements touched per line (<= L)
 };
 
-// A stage program: Stockham passes with the given radices, the per-stage
-// twiddle tables at tw + tw_off[s] (entries (r-1)*Ns + k = w_P^(r k),
-// P = Ns*R, forward sign).
-struct StageProg {
-  int L;
-  int nst;
-  int radix[FB_MAX_STAGES];
-  int tw_off[FB_MAX_STAGES];
-  const void* tw;
-};
-
 // Division of 32-bit values below 2^31 by a divisor d >= 1 known on the host:
 // with 2^s >= d > 2^(s-1) and mul = ceil(2^(31+s) / d), x/d = (x*mul) >> (31+s)
 // for every x < 2^31, as x * (mul*d - 2^(31+s)) < 2^31 * d <= 2^(31+s).
@@ -54,6 +43,18 @@ struct Divisor {
   __host__ __device__ __forceinline__
 #endif
   uint32_t quot(uint32_t x) const { return (uint32_t)(((uint64_t)x * mul) >> shift); }
+};
+
+// A stage program: Stockham passes with the given radices, the per-stage
+// twiddle tables at tw + tw_off[s] (entries (r-1)*Ns + k = w_P^(r k),
+// P = Ns*R, forward sign).
+struct StageProg {
+  int L;
+  int nst;
+  int radix[FB_MAX_STAGES];
+  int tw_off[FB_MAX_STAGES];
+  Divisor nsd[FB_MAX_STAGES];  // Ns of each stage (the generic kernel's j mod Ns)
+  const void* tw;
 };
 
 struct LineArgs {
@@ -92,9 +93,34 @@ struct LineArgs {
                         // specialised kernels store it evict-first
   uint64_t wait_ns;     // limit of a wait on the block's own asynchronous
                         // work (tensor-core products); 0: kWaitNsDefault
-  Divisor d0, d1;       // m0 and m1 (set by the tile launches; mul 0: divide
-                        // in 64 bits)
+  Divisor d0, d1;       // m0 and m1 (with_divisors; mul 0: divide in 64 bits)
 };
+
+// The launch's arguments with the reciprocals split_line divides by.
+inline LineArgs with_divisors(LineArgs a) {
+  const int64_t lim = int64_t(1) << 31;
+  if (a.nlines < lim && a.m0 < lim && a.m1 < lim) {
+    a.d0 = Divisor((uint32_t)a.m0);
+    a.d1 = Divisor((uint32_t)a.m1);
+  } else {
+    a.d0 = a.d1 = Divisor();
+  }
+  return a;
+}
+
+
+// Fill in a program's nsd from its radices.
+inline void set_stage_divisors(StageProg* p) {
+  uint32_t ns = 1;
+  for (int s = 0; s < p->nst; ++s) {
+    p->nsd[s] = Divisor(ns);
+    ns *= (uint32_t)p->radix[s];
+  }
+}
+
+// Output pairs of a radix >= 17 butterfly that one thread of the generic
+// kernel computes at most (stage_prime).
+constexpr int kPrimePairs = 16;
 
 // Shared-memory pitch (elements) of the lines of a tile block.  A warp holds
 // G lines x 32/G butterflies, and a 128-byte row of shared memory has
@@ -105,6 +131,15 @@ struct LineArgs {
 __host__ __device__ constexpr int tile_pitch(int lpad, int G, int es) {
   return lpad + ((((G >= 128 / es ? 1 : (128 / es) / G) - lpad) % (128 / es)) + (128 / es)) %
                     (128 / es);
+}
+
+// Whether the generic kernel runs a pass's lines fastest across its threads,
+// and the shared-memory pitch of its lines then.
+inline __host__ __device__ bool elem_major(const LineArgs& a) {
+  return a.ld.mode == 1 || a.st.mode == 1;
+}
+inline __host__ __device__ int line_pitch(const LineArgs& a, int es) {
+  return elem_major(a) ? tile_pitch(a.Lpad, a.G, es) : a.Lpad;
 }
 
 // Longest line whose twiddle slice a tile block stages in shared memory.

@@ -104,7 +104,7 @@ const char* last_launch_message() { return g_launch_msg; }
 
 size_t line_smem_bytes(int dtype, const LineArgs& a) {
   const size_t es = dtype == 0 ? 8 : 16;
-  return (size_t)a.G * a.Lpad * es + (size_t)4 * a.G * sizeof(int64_t);
+  return (size_t)a.G * line_pitch(a, (int)es) * es + (size_t)5 * a.G * sizeof(int64_t);
 }
 int line_max_threads() { return 512; }
 

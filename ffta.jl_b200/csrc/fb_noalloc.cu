@@ -250,6 +250,7 @@ static int noalloc_run(const void* in, void* out, int64_t n, int64_t batch, int 
   a1.prog.L = (int)N1;
   a1.prog.nst = (int)r1.size();
   for (size_t i = 0; i < r1.size(); ++i) a1.prog.radix[i] = r1[i];
+  set_stage_divisors(&a1.prog);
   a1.prog.tw = d.tables;
   a1.dir1 = a1.dir2 = dir;
   a1.tw_N = n;
@@ -273,6 +274,7 @@ static int noalloc_run(const void* in, void* out, int64_t n, int64_t batch, int 
   a2.prog.L = (int)N2;
   a2.prog.nst = (int)r2.size();
   for (size_t i = 0; i < r2.size(); ++i) a2.prog.radix[i] = r2[i];
+  set_stage_divisors(&a2.prog);
   a2.prog.tw = tw2;
   a2.dir1 = a2.dir2 = dir;
   a2.scale = 1.0;

@@ -409,28 +409,39 @@ static bool direct_ok(int64_t n, int64_t cutoff, int dtype) {
   return true;
 }
 
+// Threads per line of the generic kernel for a radix program when a thread
+// holds at most `cap` values of a stage (radices <= 16) or kPrimePairs output
+// pairs of a prime butterfly; 0 if more than line_max_threads().  Up to 32
+// threads a power of two, else whole warps.
+static int line_threads(int L, const std::vector<int>& rad, int cap) {
+  int tmin = 1, twant = 1;
+  for (int R : rad) {
+    const int nb = L / R;
+    if (R > 16) {
+      // four pairs per thread where that takes at most 256 threads
+      const int pairs = (R + 1) / 2;
+      tmin = std::max(tmin, nb * ((pairs + kPrimePairs - 1) / kPrimePairs));
+      twant = std::max(twant, nb * ((pairs + 3) / 4));
+    } else {
+      tmin = std::max(tmin, (nb + um_for(R, cap) - 1) / um_for(R, cap));
+    }
+  }
+  if (twant <= 256) tmin = std::max(tmin, twant);
+  if (tmin > line_max_threads()) return 0;
+  if (tmin > 32) return (tmin + 31) / 32 * 32;
+  int T = 1;
+  while (T < tmin) T <<= 1;
+  return T;
+}
+
 // Threads per line and the kernel variant for a radix program.
 static bool pick_threads(int L, const std::vector<int>& rad, int* T_out, int* variant_out) {
   bool big = false;
   for (int R : rad) big |= R > 16;
-  const int caps[2] = {16, 32};
-  for (int ci = 0; ci < 2; ++ci) {
-    const int cap = caps[ci];
+  for (int cap : {16, 32}) {
     if (big && cap != 16) break;
-    int tmin = 1;
-    for (int R : rad) {
-      const int nb = L / R;
-      const int need = (nb + um_for(R, cap) - 1) / um_for(R, cap);
-      tmin = std::max(tmin, need);
-    }
-    if (tmin <= line_max_threads()) {
-      int T;
-      if (tmin <= 32) {
-        T = 1;
-        while (T < tmin) T <<= 1;
-      } else {
-        T = (tmin + 31) / 32 * 32;
-      }
+    const int T = line_threads(L, rad, cap);
+    if (T) {
       *T_out = T;
       *variant_out = (cap == 32 ? 1 : 0) | (big ? 2 : 0);
       return true;
@@ -865,6 +876,7 @@ static void fill_prog(fb_plan_s* P, LineX& x, StageProg* prog) {
     prog->radix[s] = x.radices[s];
     prog->tw_off[s] = x.tw_off[s];
   }
+  set_stage_divisors(prog);
   prog->tw = tw;
 }
 
@@ -2724,7 +2736,7 @@ static const SrvShape* srv_shape(fb_server_s* S, const fb_plan_s* T, int dtype) 
   std::vector<int> rad(sh.a.prog.radix, sh.a.prog.radix + sh.a.prog.nst);
   if (!pick_threads(sh.a.prog.L, rad, &Tt, &var)) fail(FB_ERR_UNSUPPORTED, "no thread shape");
   sh.threads = Tt > 256 ? 512 : 256;
-  const size_t line_bytes = (size_t)sh.a.Lpad * elem_bytes(dtype) + 4 * sizeof(int64_t);
+  const size_t line_bytes = (size_t)sh.a.Lpad * elem_bytes(dtype) + 5 * sizeof(int64_t);
   int cls = 0;
   while (cls < 3 && line_bytes > kSmemClass[cls]) ++cls;
   int G = std::max(1, sh.threads / Tt);
@@ -2822,6 +2834,7 @@ static void srv_dispatch(fb_server_s* S) {
     a.m0 = r.batch;
     a.m1 = 1;
     a.scale = 1.0;
+    a = with_divisors(a);
     Group& g = groups[std::make_tuple(r.dtype, var, threads, cls)];
     g.descs.push_back(a);
     g.bstart.push_back(g.bstart.back() + (r.batch + G - 1) / G);
@@ -3169,15 +3182,8 @@ static std::vector<Shape> pass_shapes(const fb_plan_s* P, const Pass& p) {
     const bool em = p.a.ld.mode == 1 || p.a.st.mode == 1;
     for (int cap : {16, 32}) {
       if (big && cap == 32) continue;
-      int tmin = 1;
-      for (int R : rad) tmin = std::max(tmin, (p.a.prog.L / R + um_for(R, cap) - 1) / um_for(R, cap));
-      if (tmin > line_max_threads()) continue;
-      int T = 1;
-      if (tmin <= 32) {
-        while (T < tmin) T <<= 1;
-      } else {
-        T = (tmin + 31) / 32 * 32;
-      }
+      const int T = line_threads(p.a.prog.L, rad, cap);
+      if (!T) continue;
       const int variant = (cap == 32 ? 1 : 0) | (big ? 2 : 0);
       for (int G : gs) {
         if (em && (G & (G - 1))) continue;  // element-major tiles take powers of two
