@@ -497,9 +497,12 @@ __device__ __forceinline__ void run_prog(cplx<R>* buf, const StageProg& p, const
 // Where a pass's lines are neighbours in memory (element-major: ld.mode or
 // st.mode 1; G is a power of two) the lines run fastest across the threads,
 // g = tid mod G, and the line pitch spreads them over the banks.  The first
-// stage reads, and the last stage writes, global memory directly when that
-// order suits the access; loads of contiguous lines by an element-major
-// block go through shared memory.
+// stage reads and the last stage writes global memory directly.  Where one
+// side's lines are contiguous (the rows of a four-step's second pass) an
+// element-major block holds G lines such that a warp still covers whole
+// 32-byte sectors of each (pick_G); staging those loads through shared memory
+// instead formed the four-step twiddle element by element, 80 instructions
+// each: 23100 x 256 ComplexF32 116.9 -> 102.8 us.
 constexpr int kIdle = 1 << 29;
 
 template <typename R, int CAP, bool BIG>
@@ -535,8 +538,8 @@ __device__ __forceinline__ void line_body(const LineArgs& a, int64_t block, int 
   // direct I/O: not for the prime stages, which work in shared memory, nor
   // for an empty program (a copy)
   const bool direct = a.prog.nst > 0;
-  const bool ld = direct && (a.ld.mode == 1) == em && a.prog.radix[0] <= 16;
-  const bool st = direct && (a.st.mode == 1) == em && a.prog.radix[a.prog.nst - 1] <= 16;
+  const bool ld = direct && a.prog.radix[0] <= 16;
+  const bool st = direct && a.prog.radix[a.prog.nst - 1] <= 16;
   C* buf = sm + g * Lp;
   const R* pcs = (const R*)a.prime_cs;
   const int rad0 = direct ? a.prog.radix[0] : 1, nb0 = L / rad0;

@@ -636,7 +636,8 @@ struct fb_plan_s {
 
 namespace fb {
 
-static int pick_G(const fb_plan_s* P, int L, int T, int Lpad, bool elem_major, int64_t nlines);
+static int pick_G(const fb_plan_s* P, int L, int T, int Lpad, bool elem_major, int64_t nlines,
+                  bool mixed = false);
 static void apply_tuning(fb_plan_s* P);
 static void plan_tma(const fb_plan_s* P, Pass& p);
 static int lpad_for(int L);
@@ -929,7 +930,11 @@ static void blue_tables(fb_plan_s* P, int64_t N, int64_t M, void** pre, void** p
   *mid = chirp_spectrum(P, N, M, 1.0);
 }
 
-static int pick_G(const fb_plan_s* P, int L, int T, int Lpad, bool elem_major, int64_t nlines) {
+// Lines per block of the generic kernel.  mixed: an element-major pass with one
+// contiguous side, whose blocks take so many lines that a warp's 32/G
+// neighbouring elements of a line fill a 32-byte sector.
+static int pick_G(const fb_plan_s* P, int L, int T, int Lpad, bool elem_major, int64_t nlines,
+                  bool mixed) {
   const int es = elem_bytes(P->dtype);
   const int thr_cap = std::max(1, std::max(line_max_threads(), T) / T);
   const size_t line_bytes = (size_t)Lpad * es + 24;
@@ -940,6 +945,7 @@ static int pick_G(const fb_plan_s* P, int L, int T, int Lpad, bool elem_major, i
   int G = std::min(std::min(thr_cap, g_smem), want);
   int64_t nl = std::max<int64_t>(1, nlines);
   while (G > 1 && G / 2 >= nl) G /= 2;
+  if (mixed) G = std::min(G, es == 8 ? 8 : 16);
   if (elem_major) {
     int p = 1;
     while (p * 2 <= G) p *= 2;
@@ -1110,7 +1116,7 @@ static Axis plan_direct_axis(fb_plan_s* P, int64_t n, LineX& x, int64_t is, int6
   const bool st_em = os != 1 && !inner.empty() && inner[0].os == 1;
   p.a.ld.mode = ld_em ? 1 : 0;
   p.a.st.mode = st_em ? 1 : 0;
-  p.a.G = pick_G(P, x.L, x.T, p.a.Lpad, ld_em || st_em, nl);
+  p.a.G = pick_G(P, x.L, x.T, p.a.Lpad, ld_em || st_em, nl, ld_em != st_em);
   ax.kind = x.kind == 0 ? "DIRECT" : "BLUE1";
   // Contiguous lines at one batch stride: the specialised direct-I/O kernel.
   const FastFn* ff = nullptr;
@@ -1266,7 +1272,7 @@ static Axis plan_four_axis(fb_plan_s* P, int64_t N, int64_t N1, int64_t N2, Line
   }
   p1.a.G = pick_G(P, x1.L, x1.T, p1.a.Lpad, true, p1.a.nlines);
   p2.a.G = pick_G(P, x2.L, x2.T, p2.a.Lpad, p2.a.ld.mode == 1 || p2.a.st.mode == 1,
-                  p2.a.nlines);
+                  p2.a.nlines, p2.a.ld.mode != p2.a.st.mode);
   std::ostringstream w1, w2;
   w1 << "FOUR" << (tmode ? "T" : "") << ".1(N1=" << N1 << (x1.kind ? " blue" : "")
      << " L=" << x1.L << " T=" << x1.T << " G=" << p1.a.G << ")";
