@@ -1749,7 +1749,7 @@ static void execute_plan(fb_plan_s* P, const void* in, void* out, cudaStream_t s
   }
 }
 
-static int guard(const std::function<void()>& f) {
+template <class Fn> static int guard(const Fn& f) {
   try {
     f();
     g_last_error.clear();

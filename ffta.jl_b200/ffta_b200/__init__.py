@@ -81,9 +81,21 @@ def version() -> str:
 
 
 # ------------------------------------------------------------------ arrays
+# torch.Tensor and torch._C, once a tensor has been seen (its user imports torch)
+_Tensor = None
+_C = None
+
+
 def _is_torch(x) -> bool:
+    global _Tensor, _C
     t = type(x)
-    return t.__module__.startswith("torch") and t.__name__ == "Tensor"
+    if t is _Tensor:
+        return True
+    if _Tensor is None and t.__module__.startswith("torch") and t.__name__ == "Tensor":
+        _C = _torch()._C
+        _Tensor = t
+        return True
+    return False
 
 
 def _torch():
@@ -355,29 +367,31 @@ def size(p: FFTAPlan_cx, i=None):
     return p.size(i)
 
 
+def _layout(x):
+    """What a plan's checks and schedule depend on in a CUDA tensor: shape,
+    strides, element type and device.  None for anything else, lazily
+    conjugated or negated views included."""
+    if not _is_torch(x) or not x.is_cuda or x.is_conj() or x.is_neg():
+        return None
+    return x.shape, x.stride(), x.dtype, x.get_device()
+
+
 def _fast_key(y, x):
-    """Layout key of two complex CUDA tensors (shapes, strides, type,
-    devices), or None for anything else."""
-    if not (_is_torch(x) and _is_torch(y)):
+    """Layouts of two complex CUDA tensors of one element type, or None."""
+    a, b = _layout(x), _layout(y)
+    if a is None or b is None or a[2] is not b[2] or not a[2].is_complex:
         return None
-    dt = x.dtype
-    if dt is not y.dtype or not dt.is_complex or not x.is_cuda or not y.is_cuda:
-        return None
-    if x.is_conj() or x.is_neg() or y.is_conj() or y.is_neg():
-        return None
-    return (x.shape, x.stride(), y.shape, y.stride(), dt, x.device.index, y.device.index)
+    return a, b
 
 
 def _execute_device(h, x, y):
     """fb_execute on the current stream of x's device."""
-    torch = _torch()
-    dev = x.device
-    stream = torch.cuda.current_stream(dev).cuda_stream
-    args = (h, ctypes.c_void_p(x.data_ptr()), ctypes.c_void_p(y.data_ptr()), ctypes.c_void_p(stream))
-    if dev.index == torch.cuda.current_device():
+    dev = x.get_device()
+    args = h, x.data_ptr(), y.data_ptr(), _C._cuda_getCurrentRawStream(dev)
+    if dev == _C._cuda_getDevice():
         _check(lib.fb_execute(*args))
     else:
-        with torch.cuda.device(dev):
+        with _torch().cuda.device(dev):
             _check(lib.fb_execute(*args))
 
 
@@ -529,6 +543,9 @@ class FFTAPlan_re:
         self.BLUESTEIN_CUTOFF = cutoff
         self.scale = scale
         self._cplans = {}
+        # layouts of device tensors that passed every check of __mul__ without
+        # a copy -> (C plan, output's memory shape, element type, dim order)
+        self._fast = {}
 
     def size(self, i=None):
         """Base.size (src/plan.jl:36-47): the real length first."""
@@ -578,6 +595,13 @@ class FFTAPlan_re:
         return h
 
     def __mul__(self, x):
+        fk = _layout(x)
+        f = self._fast.get(fk) if fk is not None else None
+        if f is not None:  # laid out like an earlier array: the checks depend on nothing else
+            h, shape, odt, order = f
+            y = x.new_empty(shape, dtype=odt)
+            _execute_device(h, x, y)
+            return y.permute(order)
         kind = _real_kind(x)
         vec = x.ndim == 1
         what = "vectors" if vec else "arrays"
@@ -629,12 +653,16 @@ class FFTAPlan_re:
                 odt = torch.complex64 if self._prec == "f32" else torch.complex128
             else:
                 odt = torch.float32 if self._prec == "f32" else torch.float64
-            y = torch.empty(tuple(reversed(out_dims)), dtype=odt, device=x.device)
+            shape, order = tuple(reversed(out_dims)), tuple(range(len(out_dims) - 1, -1, -1))
+            y = torch.empty(shape, dtype=odt, device=x.device)
             stream = torch.cuda.current_stream(x.device).cuda_stream
             with torch.cuda.device(x.device):
                 _check(lib.fb_execute(h, ctypes.c_void_p(xc.data_ptr()),
                                       ctypes.c_void_p(y.data_ptr()), ctypes.c_void_p(stream)))
-            return y.permute(tuple(range(y.ndim - 1, -1, -1)))
+            fk = _layout(x)
+            if fk is not None and xc.data_ptr() == x.data_ptr():
+                self._fast[fk] = h, shape, odt, order
+            return y.permute(order)
         if complex_out:
             odt = np.complex64 if self._prec == "f32" else np.complex128
         else:
