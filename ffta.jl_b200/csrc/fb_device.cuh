@@ -13,6 +13,43 @@
 
 namespace fb {
 
+// ------------------------------------------------------------- launches
+// Launch k so that its blocks may become resident while the stream's previous
+// kernel drains (programmatic stream serialization): the launch and the
+// block's index arithmetic overlap that kernel's end.  k must call
+// grid_wait() in every thread before it touches memory another kernel reads
+// or writes.  One B200, before -> after: 1000 x 1000 ComplexF32 18.4 -> 14.4
+// us, 65537 x 16 81.4 -> 73.4, 4096 x 16384 206.4 -> 195.7, 2^16 x 1 10.3 ->
+// 8.1.
+//
+// early = false: an ordinary launch.
+template <class... P, class... A>
+inline cudaError_t launch_overlapped(bool early, void (*k)(P...), dim3 grid, dim3 block,
+                                     size_t smem, cudaStream_t s, A&&... args) {
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = early ? 1 : 0;
+  cudaLaunchConfig_t c = {};
+  c.gridDim = grid;
+  c.blockDim = block;
+  c.dynamicSmemBytes = smem;
+  c.stream = s;
+  c.attrs = &at;
+  c.numAttrs = 1;
+  return cudaLaunchKernelEx(&c, k, static_cast<A&&>(args)...);
+}
+// Wait until the stream's previous kernels have completed and their writes are
+// visible.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Let the stream's next kernel be launched once every block has come here (or
+// ended); it waits in its own grid_wait.  Called where a block begins its last
+// stage: released at their start, blocks of the next launch of less than a
+// wave crowded onto the SMs that this one left free (three-pass Bluestein
+// 449699 ComplexF64 61.4 -> 70.8 us).
+__device__ __forceinline__ void grid_release() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // ------------------------------------------------------------ scalar ops
 template <typename R> struct Sc;
 template <> struct Sc<float> {

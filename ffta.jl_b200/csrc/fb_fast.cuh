@@ -25,6 +25,7 @@
 // order of stages -- is exactly that of the generic line kernel
 // (fb_line.cuh), so all of them produce the same bits for the same length.
 #pragma once
+#include <atomic>
 #include <cstdio>
 #include <cstring>
 #include <type_traits>
@@ -401,6 +402,7 @@ __device__ __forceinline__ void fast_stage(cplx<R>* buf, const In& in, const Out
   constexpr bool GOUT = S == RL::n - 1 && !std::is_same<Out, SmemIO>::value;
   static_assert(!TC || (S == 0 && RAD == 16 && UM == 1 && nb == T && std::is_same<R, float>::value),
                 "the tensor-core stage is a first radix-16 stage, one butterfly per thread");
+  if constexpr (GOUT) grid_release();
   cplx<R> v[UM][RAD];
 #pragma unroll
   for (int q = 0; q < UM; ++q) {
@@ -512,6 +514,7 @@ __global__ void __launch_bounds__(DirectBounds<R, T>::threads, DirectBounds<R, T
   const int64_t l = ok ? line : 0;
   const C* gin = (const C*)a.in + l * a.idist;
   C* gout = (C*)a.out + l * a.odist;
+  grid_wait();
   if (a.ndesc > 0) {
     // grouped launch: find the request owning this line (binary search)
     int lo = 0, hi = a.ndesc - 1;
@@ -579,6 +582,7 @@ __global__ void __launch_bounds__(T, StreamBounds<R, RL, T>::min_blocks)
   const int64_t nmine = first < a.nlines ? (a.nlines - 1 - first) / step + 1 : 0;
   const C* gin = (const C*)a.in;
   C* gout = (C*)a.out;
+  grid_wait();
   if (u == 0) {
     for (int b = 0; b < NBUF; ++b) mbar_init(bar + b, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -718,6 +722,7 @@ __global__ void __launch_bounds__(TileThreads<R, T, MID>::value,
       lb[3 * G + g] = q0 | (a.tw_level ? q1 : q0) << 32;  // both below 2^31 (use_tile)
     }
   }
+  grid_wait();
   __syncthreads();
   const C* tw = (const C*)a.prog.tw;
   const R* pcs = (const R*)a.prime_cs;
@@ -832,9 +837,11 @@ __global__ void __launch_bounds__(DirectBounds<R, T>::threads, DirectBounds<R, T
   const C* __restrict__ wk = (const C*)a.wk;
   const R h = R(0.5), sc = (R)a.scale;
   const bool cs = a.st_stream != 0;
+  grid_wait();
   if constexpr (DIR < 0) {
     const DirectIn<R> in{(const C*)((const R*)a.in + l * a.idist), ok};
     fast_prog<R, -1, RL, T>(buf, in, SmemIO{}, tw, pcs, u);
+    grid_release();
     if (!ok) return;  // (no barrier follows)
     C* o = (C*)a.out + l * a.odist;
     for (int k = u; k <= L / 2; k += T) {
@@ -952,6 +959,7 @@ __global__ void __launch_bounds__(TileThreads<R, T, false>::value,
       tma_load_4d(dst + (size_t)r * box_bytes, &tm, (int)(q0 * q.units), r * q.boxr, (int)q1,
                   (int)q2, bar + b);
   };
+  grid_wait();
   if (tid == 0) {
     for (int b = 0; b < q.nbuf; ++b) mbar_init(bar + b, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -1040,6 +1048,7 @@ __global__ void __launch_bounds__(T, TcShape<RL, T>::direct_blocks)
   uint64_t* bar = (uint64_t*)(b + tc::kTcTableBytes);
   uint32_t* slot = (uint32_t*)(bar + 1);
   const int u = threadIdx.x;
+  grid_wait();
   const tc::TcCtx c =
       tc::tc_begin(smraw, b, bar, slot,
                    (const unsigned char*)a.tcb + (DIR < 0 ? 0 : tc::kTcTableBytes), a.err, u, T,
@@ -1074,6 +1083,7 @@ __global__ void __launch_bounds__(512, 2) fast_tc_tile_kernel(const LineArgs a) 
     lb[2 * G + g] = q0 * a.st.s0 + q1 * a.st.s1 + q2 * a.st.s2;
     lb[3 * G + g] = a.tw_level ? q1 : q0;
   }
+  grid_wait();
   // (tc_begin's barrier publishes lb)
   const tc::TcCtx c = tc::tc_begin(
       smraw, b, bar, slot, (const unsigned char*)a.tcb + (a.dir1 < 0 ? 0 : tc::kTcTableBytes),
@@ -1111,6 +1121,27 @@ template <typename K> static cudaError_t tc_check_columns(K k, int threads, size
 }
 
 // ---------------------------------------------------------- launching
+// Blocks of a kernel one SM holds, remembered for the launch shape last asked
+// for (threads, shared memory, device in one word, so concurrent callers see
+// one shape or the other).
+struct Occupancy {
+  std::atomic<uint64_t> last{0};
+  template <class... P> int blocks(void (*k)(P...), int threads, size_t smem) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev >= 256) return 0;
+    const uint64_t key = (uint64_t)smem << 32 | (uint64_t)threads << 16 | (uint64_t)dev << 8;
+    const uint64_t seen = last.load(std::memory_order_relaxed);
+    if ((seen & ~uint64_t(255)) == key && (seen & 255)) return (int)(seen & 255);
+    int n = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, threads, smem) != cudaSuccess) return 0;
+    last.store(key | (uint64_t)(n & 255), std::memory_order_relaxed);
+    return n;
+  }
+};
+
+
+constexpr int kSms = 148;
+
 // Raise a kernel's dynamic shared-memory limit when a launch needs more than
 // the default 48 KB.  `set` is the caller's per-kernel, per-device record.
 template <typename K> static cudaError_t configure(K k, size_t smem, int* set) {
@@ -1154,8 +1185,7 @@ template <typename R, class RL, int T> struct FastEntry {
     }
     const int64_t nblk = (a.nlines + a.G - 1) / a.G;
     if (nblk <= 0) return cudaSuccess;
-    k<<<dim3((unsigned)nblk), dim3(T, a.G), smem, s>>>(a);
-    e = cudaGetLastError();
+    e = launch_overlapped(true, k, dim3((unsigned)nblk), dim3(T, a.G), smem, s, a);
     if (e != cudaSuccess) launch_failure(k, "direct launch", L, T, a.G, smem, e);
     return e;
   }
@@ -1188,8 +1218,7 @@ template <typename R, class RL, int T> struct FastEntry {
       }
       if (a.nlines <= 0) return cudaSuccess;
       const int64_t nblk = a.nlines < per_sm ? a.nlines : per_sm;
-      k<<<dim3((unsigned)nblk), dim3(T), smem, s>>>(a);
-      e = cudaGetLastError();
+      e = launch_overlapped(true, k, dim3((unsigned)nblk), dim3(T), smem, s, a);
       if (e != cudaSuccess) launch_failure(k, "stream launch", L, T, 1, smem, e);
       return e;
     }
@@ -1216,8 +1245,7 @@ template <typename R, class RL, int T> struct FastEntry {
       }
       const int64_t nblk = (a.nlines + a.G - 1) / a.G;
       if (nblk <= 0) return cudaSuccess;
-      k<<<dim3((unsigned)nblk), dim3(T, a.G), smem, s>>>(a);
-      e = cudaGetLastError();
+      e = launch_overlapped(true, k, dim3((unsigned)nblk), dim3(T, a.G), smem, s, a);
       if (e != cudaSuccess) launch_failure(k, "real launch", L, T, a.G, smem, e);
       return e;
     }
@@ -1253,9 +1281,8 @@ template <typename R, class RL, int T> struct FastEntry {
       if (q.ntiles <= 0) return cudaSuccess;
       const int64_t cap = (int64_t)per_sm * nsm;
       const int64_t nblk = q.ntiles < cap ? q.ntiles : cap;
-      k<<<dim3((unsigned)nblk), dim3(a.G, T), smem, s>>>(with_divisors(a),
-                                                         *(const CUtensorMap*)tmap, q);
-      e = cudaGetLastError();
+      e = launch_overlapped(true, k, dim3((unsigned)nblk), dim3(a.G, T), smem, s, with_divisors(a),
+                            *(const CUtensorMap*)tmap, q);
       if (e != cudaSuccess) launch_failure(k, "tensor-copy tile launch", L, T, a.G, smem, e);
       return e;
     }
@@ -1278,8 +1305,7 @@ template <typename R, class RL, int T> struct FastEntry {
         return e;
       }
       if (a.nlines <= 0) return cudaSuccess;
-      k<<<dim3((unsigned)a.nlines), dim3(T), smem, s>>>(a);
-      e = cudaGetLastError();
+      e = launch_overlapped(true, k, dim3((unsigned)a.nlines), dim3(T), smem, s, a);
       if (e != cudaSuccess) launch_failure(k, "tensor-core direct launch", L, T, 1, smem, e);
       return e;
     }
@@ -1305,14 +1331,14 @@ template <typename R, class RL, int T> struct FastEntry {
       }
       const int64_t nblk = (a.nlines + a.G - 1) / a.G;
       if (nblk <= 0) return cudaSuccess;
-      k<<<dim3((unsigned)nblk), dim3(a.G, T), smem, s>>>(with_divisors(a));
-      e = cudaGetLastError();
+      e = launch_overlapped(true, k, dim3((unsigned)nblk), dim3(a.G, T), smem, s, with_divisors(a));
       if (e != cudaSuccess) launch_failure(k, "tensor-core tile launch", L, T, a.G, smem, e);
       return e;
     }
   }
   static cudaError_t launch_tile(const LineArgs& a, cudaStream_t s) {
     static int set_plain[64] = {0}, set_mid[64] = {0}, set_full[64] = {0};
+    static Occupancy op, om;
     const size_t smem = (size_t)a.G * tile_pitch(LPAD, a.G, (int)sizeof(cplx<R>)) * sizeof(cplx<R>) +
                         (size_t)a.G * 4 * sizeof(int64_t) +
                         (stages_twiddles(a, L) ? (size_t)L * sizeof(cplx<R>) : 0);
@@ -1333,8 +1359,22 @@ template <typename R, class RL, int T> struct FastEntry {
     }
     const int64_t nblk = (a.nlines + a.G - 1) / a.G;
     if (nblk <= 0) return cudaSuccess;
-    k<<<dim3((unsigned)nblk), dim3(a.G, T), smem, s>>>(with_divisors(a));
-    e = cudaGetLastError();
+    // Blocks launched early go to the SMs the previous kernel has left, as many
+    // as fit, while a grid that starts on an idle device is dealt out evenly.
+    // Passes of less than a wave that fill the SMs (256 threads or more per SM)
+    // and could crowd therefore start after the previous kernel: a Bluestein
+    // middle pass of which more blocks fit an SM than its even share (449699
+    // ComplexF64, 243 blocks, three fit: 75.8 us early, 64.2 not), and the rows
+    // of a four-step where twice the even share fits (2^20 x 1 ComplexF32, 1024
+    // blocks of 64: 25.3 early, 19.6 not).  Lighter ones are bound by latency
+    // and start early (2^18 x 1, 512 blocks of 32: 10.4 early, 12.3 not; middle
+    // pass of 8761 x 3, 432 blocks of 8: 38.4 early, 40.9 not).
+    bool early = true;
+    const int64_t share = (nblk + kSms - 1) / kSms;
+    if ((mid || (a.plain_io && a.ld.mode == 0)) && share * a.G * T >= 256)
+      early = (mid ? om : op).blocks(k, a.G * T, smem) < (mid ? share + 1 : 2 * share);
+    e = launch_overlapped(early, k, dim3((unsigned)nblk), dim3(a.G, T),
+                          smem, s, with_divisors(a));
     if (e != cudaSuccess) launch_failure(k, "tile launch", L, T, a.G, smem, e);
     return e;
   }

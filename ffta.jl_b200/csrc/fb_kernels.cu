@@ -345,6 +345,8 @@ struct RealGeom {
 template <typename R>
 __global__ void k_real_to_complex(const R* __restrict__ in, cplx<R>* __restrict__ out,
                                   int64_t count) {
+  grid_release();
+  grid_wait();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < count;
        i += (int64_t)gridDim.x * blockDim.x)
     out[i] = Sc<R>::mk(in[i], R(0));
@@ -353,6 +355,8 @@ __global__ void k_real_to_complex(const R* __restrict__ in, cplx<R>* __restrict_
 template <typename R>
 __global__ void k_complex_to_real(const cplx<R>* __restrict__ in, R* __restrict__ out,
                                   int64_t count) {
+  grid_release();
+  grid_wait();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < count;
        i += (int64_t)gridDim.x * blockDim.x)
     out[i] = in[i].x;
@@ -363,6 +367,8 @@ __global__ void k_complex_to_real(const cplx<R>* __restrict__ in, R* __restrict_
 template <typename R>
 __global__ void k_extract_half(const cplx<R>* __restrict__ in, cplx<R>* __restrict__ out,
                                Dims half, int64_t n, int64_t count) {
+  grid_release();
+  grid_wait();
   for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < count;
        q += (int64_t)gridDim.x * blockDim.x) {
     int64_t t = q;
@@ -378,6 +384,8 @@ __global__ void k_extract_half(const cplx<R>* __restrict__ in, cplx<R>* __restri
 template <typename R>
 __global__ void k_herm_extend(const cplx<R>* __restrict__ x, cplx<R>* __restrict__ z, RealGeom g,
                               int64_t total) {
+  grid_release();
+  grid_wait();
   for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < total;
        q += (int64_t)gridDim.x * blockDim.x) {
     // offsets of the entry itself and of its mirror image in x
@@ -397,7 +405,7 @@ __global__ void k_herm_extend(const cplx<R>* __restrict__ x, cplx<R>* __restrict
 }
 
 // The split and the merge of the half-length algorithm (fast_real_kernel's
-// arithmetic) as passes of their own, around a complex plan of length L = n/2
+// formulas) as passes of their own, around a complex plan of length L = n/2
 // on the real line read as L complex values: for halves without a one-kernel
 // real transform.  Thread (k, line) handles the outputs k and L-k; a thread
 // keeps w^k for all its lines.  Bound by memory: one read and one write of
@@ -409,6 +417,8 @@ __global__ void __launch_bounds__(256)
                 const cplx<R>* __restrict__ wk, int L, int64_t lines, R scale) {
   typedef cplx<R> C;
   typedef Sc<R> S;
+  grid_release();
+  grid_wait();
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k > L / 2) return;
   const C w = __ldg(wk + k);
@@ -427,12 +437,12 @@ __global__ void __launch_bounds__(256)
       const C B = __ldcs(z + (L - k));
       const C xx = S::mk(S::mul(h, S::add(A.x, B.x)), S::mul(h, S::sub(A.y, B.y)));
       const C xy = S::mk(S::mul(h, S::add(B.y, A.y)), S::mul(h, S::sub(B.x, A.x)));
-      const C wxy = cmul<R>(w, xy);
-      o[k] = cscale<R>(cadd<R>(xx, wxy), scale);
-      if (k != L - k) {
-        const C d = csub<R>(xx, wxy);
-        o[L - k] = cscale<R>(S::mk(d.x, -d.y), scale);
-      }
+      // XX + w XY and conj(XX - w XY), two roundings each
+      o[k] = cscale<R>(S::mk(S::fma(w.x, xy.x, S::fma(-w.y, xy.y, xx.x)),
+                             S::fma(w.x, xy.y, S::fma(w.y, xy.x, xx.y))), scale);
+      if (k != L - k)
+        o[L - k] = cscale<R>(S::mk(S::fma(-w.x, xy.x, S::fma(w.y, xy.y, xx.x)),
+                                   -S::fma(-w.x, xy.y, S::fma(-w.y, xy.x, xx.y))), scale);
     } else {
       const C* y = in + l * (L + 1);
       C* z = out + l * L;
@@ -443,13 +453,12 @@ __global__ void __launch_bounds__(256)
       }
       const C xx = S::mk(S::add(A.x, B.x), S::sub(A.y, B.y));
       const C dd = S::mk(S::sub(A.x, B.x), S::add(A.y, B.y));
-      const C xy = cmulc<R>(dd, w);
-      const C ixy = S::mk(-xy.y, xy.x);
-      z[k] = cadd<R>(xx, ixy);
-      if (k != L - k) {
-        const C d = csub<R>(xx, ixy);
-        z[L - k] = S::mk(d.x, -d.y);
-      }
+      // XX + i conj(w) DD and conj(XX - i conj(w) DD), two roundings each
+      z[k] = S::mk(S::fma(-w.x, dd.y, S::fma(w.y, dd.x, xx.x)),
+                   S::fma(w.x, dd.x, S::fma(w.y, dd.y, xx.y)));
+      if (k != L - k)
+        z[L - k] = S::mk(S::fma(w.x, dd.y, S::fma(-w.y, dd.x, xx.x)),
+                         -S::fma(-w.x, dd.x, S::fma(-w.y, dd.y, xx.y)));
     }
   }
 }
@@ -466,9 +475,8 @@ static cudaError_t real_half_t(bool split, const void* in, void* out, const void
   const int64_t gy = std::min<int64_t>(std::min<int64_t>(want, 65535),
                                        std::max<int64_t>(1, 16 * 148 / gx));
   auto k = split ? k_real_half<R, true> : k_real_half<R, false>;
-  k<<<dim3((unsigned)gx, (unsigned)gy), block, 0, s>>>((const C*)in, (C*)out, (const C*)wk, L,
-                                                      lines, (R)scale);
-  return cudaGetLastError();
+  return launch_overlapped(true, k, dim3((unsigned)gx, (unsigned)gy), block, 0, s, (const C*)in, (C*)out,
+                           (const C*)wk, L, lines, (R)scale);
 }
 cudaError_t real_half(int dtype, bool split, const void* in, void* out, const void* wk, int L,
                       int64_t lines, double scale, cudaStream_t s) {
@@ -480,21 +488,17 @@ cudaError_t real_half(int dtype, bool split, const void* in, void* out, const vo
 cudaError_t real_to_complex(int dtype, const void* in, void* out, int64_t count, cudaStream_t s) {
   if (count <= 0) return cudaSuccess;
   if (dtype == 0)
-    k_real_to_complex<float><<<grid_for(count), 256, 0, s>>>((const float*)in, (float2*)out, count);
+    return launch_overlapped(true, k_real_to_complex<float>, grid_for(count), 256, 0, s, (const float*)in, (float2*)out, count);
   else
-    k_real_to_complex<double><<<grid_for(count), 256, 0, s>>>((const double*)in, (double2*)out,
-                                                               count);
-  return cudaGetLastError();
+    return launch_overlapped(true, k_real_to_complex<double>, grid_for(count), 256, 0, s, (const double*)in, (double2*)out, count);
 }
 
 cudaError_t complex_to_real(int dtype, const void* in, void* out, int64_t count, cudaStream_t s) {
   if (count <= 0) return cudaSuccess;
   if (dtype == 0)
-    k_complex_to_real<float><<<grid_for(count), 256, 0, s>>>((const float2*)in, (float*)out, count);
+    return launch_overlapped(true, k_complex_to_real<float>, grid_for(count), 256, 0, s, (const float2*)in, (float*)out, count);
   else
-    k_complex_to_real<double><<<grid_for(count), 256, 0, s>>>((const double2*)in, (double*)out,
-                                                              count);
-  return cudaGetLastError();
+    return launch_overlapped(true, k_complex_to_real<double>, grid_for(count), 256, 0, s, (const double2*)in, (double*)out, count);
 }
 
 cudaError_t extract_half(int dtype, const void* in, void* out, int64_t pre, int64_t n, int64_t h,
@@ -504,12 +508,9 @@ cudaError_t extract_half(int dtype, const void* in, void* out, int64_t pre, int6
   const int64_t hd[3] = {pre, h, post};
   const Dims half = make_dims(3, hd);
   if (dtype == 0)
-    k_extract_half<float><<<grid_for(count), 256, 0, s>>>((const float2*)in, (float2*)out, half, n,
-                                                          count);
+    return launch_overlapped(true, k_extract_half<float>, grid_for(count), 256, 0, s, (const float2*)in, (float2*)out, half, n, count);
   else
-    k_extract_half<double><<<grid_for(count), 256, 0, s>>>((const double2*)in, (double2*)out, half,
-                                                           n, count);
-  return cudaGetLastError();
+    return launch_overlapped(true, k_extract_half<double>, grid_for(count), 256, 0, s, (const double2*)in, (double2*)out, half, n, count);
 }
 
 cudaError_t herm_extend(int dtype, const void* x, void* z, int rank, const int64_t* dims, int r0,
@@ -524,16 +525,17 @@ cudaError_t herm_extend(int dtype, const void* x, void* z, int rank, const int64
   for (int d = 0; d < rank; ++d) total *= dims[d];
   if (total <= 0) return cudaSuccess;
   if (dtype == 0)
-    k_herm_extend<float><<<grid_for(total), 256, 0, s>>>((const float2*)x, (float2*)z, g, total);
+    return launch_overlapped(true, k_herm_extend<float>, grid_for(total), 256, 0, s, (const float2*)x, (float2*)z, g, total);
   else
-    k_herm_extend<double><<<grid_for(total), 256, 0, s>>>((const double2*)x, (double2*)z, g, total);
-  return cudaGetLastError();
+    return launch_overlapped(true, k_herm_extend<double>, grid_for(total), 256, 0, s, (const double2*)x, (double2*)z, g, total);
 }
 
 // out[sum_d k_d * os[d]] = in[sum_d k_d * is[d]] for every index (k_d < dims[d]):
 // a strided copy that moves an array between two layouts (rank <= 8).
 template <typename E>
 __global__ void k_permute(const E* __restrict__ in, E* __restrict__ out, PermCopy p, Dims dims) {
+  grid_release();
+  grid_wait();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < p.count;
        i += (int64_t)gridDim.x * blockDim.x) {
     int64_t t = i, oi = 0, oo = 0;
@@ -551,12 +553,11 @@ cudaError_t permute_copy(int elem_bytes, const void* in, void* out, const PermCo
   if (p.count <= 0) return cudaSuccess;
   const Dims dims = make_dims(p.rank, p.dims);
   switch (elem_bytes) {
-    case 4: k_permute<float><<<grid_for(p.count), 256, 0, s>>>((const float*)in, (float*)out, p, dims); break;
-    case 8: k_permute<float2><<<grid_for(p.count), 256, 0, s>>>((const float2*)in, (float2*)out, p, dims); break;
-    case 16: k_permute<double2><<<grid_for(p.count), 256, 0, s>>>((const double2*)in, (double2*)out, p, dims); break;
+    case 4: return launch_overlapped(true, k_permute<float>, grid_for(p.count), 256, 0, s, (const float*)in, (float*)out, p, dims);
+    case 8: return launch_overlapped(true, k_permute<float2>, grid_for(p.count), 256, 0, s, (const float2*)in, (float2*)out, p, dims);
+    case 16: return launch_overlapped(true, k_permute<double2>, grid_for(p.count), 256, 0, s, (const double2*)in, (double2*)out, p, dims);
     default: return cudaErrorInvalidValue;
   }
-  return cudaGetLastError();
 }
 
 cudaError_t gen_prime_tables(void* f32tab, void* f64tab, cudaStream_t s) {

@@ -290,6 +290,7 @@ __device__ __forceinline__ void stage(cplx<R>* buf, int L, int Ns, Divisor nsd,
   for (int q = 0; q < UM; ++q)
 #pragma unroll
     for (int r = 0; r < RAD; ++r) v[q][r] = Sc<R>::mk(R(0), R(0));
+  if (st) grid_release();
   if (ld) {
     const GenIn<R> in = io.input(g);
 #pragma unroll
@@ -505,9 +506,10 @@ __device__ __forceinline__ void run_prog(cplx<R>* buf, const StageProg& p, const
 // each: 23100 x 256 ComplexF32 116.9 -> 102.8 us.
 constexpr int kIdle = 1 << 29;
 
-template <typename R, int CAP, bool BIG>
+template <typename R, int CAP, bool BIG, bool OVERLAPPED>
 __device__ __forceinline__ void line_body(const LineArgs& a, int64_t block, int u, int g, int tid,
                                           unsigned char* smraw) {
+  // (OVERLAPPED: launched by launch_overlapped)
   typedef cplx<R> C;
   C* sm = (C*)smraw;
   const int T = a.T, G = a.G, L = a.prog.L;
@@ -533,6 +535,7 @@ __device__ __forceinline__ void line_body(const LineArgs& a, int64_t block, int 
         (int64_t)min(present_count(a.ld.vn, a.ld.ves, l0 * a.ld.vls, ok), ok ? a.ld.count : 0) |
         (int64_t)min(present_count(a.st.vn, a.st.ves, l0 * a.st.vls, ok), ok ? a.st.count : 0) << 32;
   }
+  if constexpr (OVERLAPPED) grid_wait();
   __syncthreads();
   const LineCtx<R> io{a, lb};
   // direct I/O: not for the prime stages, which work in shared memory, nor
@@ -576,6 +579,7 @@ __device__ __forceinline__ void line_body(const LineArgs& a, int64_t block, int 
     }
   }
   if (!st) {
+    grid_release();
     if (a.st.mode == 1 || !em) {
       const GenOut<R> dst = io.output(g);
       for (int i = u; i < L; i += T) dst.one(i, buf[padi(i)]);
@@ -598,7 +602,7 @@ template <typename R, int CAP, bool BIG>
 __global__ void __launch_bounds__(512, LineBounds<R, CAP, BIG>::min_blocks) line_kernel(const __grid_constant__ LineArgs a) {
   extern __shared__ __align__(16) unsigned char smraw[];
   const int u = threadIdx.x, g = threadIdx.y;
-  line_body<R, CAP, BIG>(a, blockIdx.x, u, g, g * a.T + u, smraw);
+  line_body<R, CAP, BIG, true>(a, blockIdx.x, u, g, g * a.T + u, smraw);
 }
 
 // Work-descriptor launch: many line transforms -- different lengths,
@@ -629,7 +633,7 @@ __global__ void __launch_bounds__(512, LineBounds<R, CAP, BIG>::min_blocks)
   const bool active = (int)threadIdx.x < nthr;
   const int u = active ? (int)threadIdx.x % sa.T : kIdle;
   const int g = active ? (int)threadIdx.x / sa.T : 0;
-  line_body<R, CAP, BIG>(sa, sblock, u, g, active ? (int)threadIdx.x : nthr, smraw);
+  line_body<R, CAP, BIG, false>(sa, sblock, u, g, active ? (int)threadIdx.x : nthr, smraw);
 }
 
 }  // namespace fb

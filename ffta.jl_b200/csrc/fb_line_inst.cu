@@ -23,8 +23,8 @@ cudaError_t FB_LAUNCH(const LineArgs& a, size_t smem, cudaStream_t s) {
   const int64_t nblk = (a.nlines + a.G - 1) / a.G;
   if (nblk <= 0) return cudaSuccess;
   dim3 grid((unsigned)nblk), block(a.T, a.G);
-  line_kernel<FB_R, FB_CAP, FB_BIG><<<grid, block, smem, s>>>(with_divisors(a));
-  return cudaGetLastError();
+  return launch_overlapped(true, line_kernel<FB_R, FB_CAP, FB_BIG>, grid, block, smem, s,
+                           with_divisors(a));
 }
 
 // Launch ndesc descriptors (device arrays) as one grid of `nblocks` blocks of
