@@ -132,11 +132,6 @@ template <typename R> __device__ __forceinline__ void store(cplx<R>* p, cplx<R> 
   else
     *p = v;
 }
-// p + r*step elements: a 32 x 32 -> 64 bit product added to the address.
-template <typename C> __device__ __forceinline__ C* step_ptr(C* p, int step, int r) {
-  return (C*)((uintptr_t)p + (uint64_t)((int64_t)step * (int64_t)(r * (int)sizeof(C))));
-}
-
 template <typename R> struct DirectIn {
   const cplx<R>* __restrict__ g;
   bool ok;

@@ -110,8 +110,27 @@ struct GenSlots {
 // One line's input or output in global memory.  `cnt` elements are present
 // (absent ones load as zero and are not stored); `mul` (the chirp) is read
 // at mul + i*ves, the four-step twiddle at tab + i*tab_es, the line's offset
-// included in both.
-template <typename R> struct GenIn {
+// included in both.  LEAN (LineArgs::plain_io): every element present, no
+// chirp and no root tables, 32-bit strides; a twiddle on the loads is
+// tw_elem's product instead of the entry itself.  What a pass rarely has is
+// applied to the registers in loops of its own, so the straight code between
+// loads and stores stays short: with the tests inside the unrolled loops a
+// quarter of the kernel's stalls were instruction fetches (no_instruction 3.5
+// of 14 cycles per issue).  One B200, before -> after: 6240 x 6 ComplexF32 14.9
+// -> 10.6 us, 231 x 3000 11.4 -> 8.8, 176 x 1728 x 5 ComplexF64 40.9 -> 34.9,
+// irfft 260 x 66 27.2 -> 17.2.
+template <typename C> __device__ __forceinline__ C* step_ptr(C* p, int step, int r) {
+  // p + r*step elements: a 32 x 32 -> 64 bit product added to the address
+  return (C*)((uintptr_t)p + (uint64_t)((int64_t)step * (int64_t)(r * (int)sizeof(C))));
+}
+template <bool LEAN, typename C>
+__device__ __forceinline__ C* row_ptr(C* p, int64_t step, int r) {
+  if constexpr (LEAN)
+    return step_ptr(p, (int)step, r);
+  else
+    return p + step * r;
+}
+template <typename R, bool LEAN> struct GenIn {
   const cplx<R>* __restrict__ base;
   int64_t es;
   int cnt;
@@ -120,41 +139,36 @@ template <typename R> struct GenIn {
   const cplx<R>* __restrict__ tab;  // twiddle on load, or null
   int64_t tab_es;
   int tw_dir;
-  bool lean;  // LineArgs::plain_io: tw_elem's product instead of the entry
 
   // inputs j + r*nb of a butterfly: every data load is issued before any
   // table load
   template <int RAD> __device__ __forceinline__ void load(int j, int nb, cplx<R>* v) const {
     const cplx<R>* p = base + j * es;
-    const int64_t step = nb * es;
 #pragma unroll
-    for (int r = 0; r < RAD; ++r) {
-      v[r] = j + r * nb < cnt ? __ldcs(p) : Sc<R>::mk(R(0), R(0));
-      p += step;
-    }
+    for (int r = 0; r < RAD; ++r)
+      v[r] = LEAN || j + r * nb < cnt ? __ldcs(row_ptr<LEAN>(p, nb * es, r))
+                                      : Sc<R>::mk(R(0), R(0));
   }
   template <int RAD> __device__ __forceinline__ void finish(int j, int nb, cplx<R>* v) const {
-    if (mul) {
+    if (!LEAN && mul) {
       const cplx<R>* p = mul + j * ves;
 #pragma unroll
-      for (int r = 0; r < RAD; ++r) {
-        if (j + r * nb < cnt) v[r] = cmul<R>(v[r], __ldg(p));
-        p += nb * ves;
-      }
+      for (int r = 0; r < RAD; ++r)
+        if (j + r * nb < cnt) v[r] = cmul<R>(v[r], __ldg(p + r * (nb * ves)));
     }
     if (!tab) return;
     const int64_t ts = nb * tab_es;
     const cplx<R>* p = tab + j * tab_es;
     auto apply = [&](int r, cplx<R> w) {
-      if (j + r * nb < cnt) v[r] = tw_dir < 0 ? cmul<R>(v[r], w) : cmulc<R>(v[r], w);
+      if (LEAN || j + r * nb < cnt) v[r] = tw_dir < 0 ? cmul<R>(v[r], w) : cmulc<R>(v[r], w);
     };
-    if (RAD >= 4 && lean) {
+    if constexpr (LEAN && RAD >= 4) {
       cplx<R> s[4];
 #pragma unroll
-      for (int c = 1; c < 4; ++c) s[c] = __ldg(tab + c * ts);
+      for (int c = 1; c < 4; ++c) s[c] = __ldg(row_ptr<LEAN>(tab, ts, c));
 #pragma unroll
       for (int a = 0; a < RAD; a += 4) {
-        const cplx<R> b = __ldg(p + a * ts);
+        const cplx<R> b = __ldg(row_ptr<LEAN>(p, ts, a));
 #pragma unroll
         for (int c = 0; c < 4; ++c)
           if (a + c < RAD) apply(a + c, c == 0 ? b : cmul<R>(b, s[c]));
@@ -162,25 +176,25 @@ template <typename R> struct GenIn {
     } else {
 #pragma unroll
       for (int r = 0; r < RAD; ++r)
-        if (j + r * nb < cnt) apply(r, __ldg(p + r * ts));
+        if (LEAN || j + r * nb < cnt) apply(r, __ldg(row_ptr<LEAN>(p, ts, r)));
     }
   }
   // element i alone (loads staged through shared memory); nb and rad of the
   // program's first stage
   __device__ __forceinline__ cplx<R> one(int i, int nb, int rad) const {
-    if (i >= cnt) return Sc<R>::mk(R(0), R(0));
+    if (!LEAN && i >= cnt) return Sc<R>::mk(R(0), R(0));
     cplx<R> v = __ldcs(base + i * es);
-    if (mul) v = cmul<R>(v, __ldg(mul + i * ves));
+    if (!LEAN && mul) v = cmul<R>(v, __ldg(mul + i * ves));
     if (tab) {
       auto at = [&](int k) { return __ldg(tab + k * tab_es); };
-      const cplx<R> w = lean ? tw_elem<R>(at, i, nb, rad) : at(i);
+      const cplx<R> w = LEAN ? tw_elem<R>(at, i, nb, rad) : at(i);
       v = tw_dir < 0 ? cmul<R>(v, w) : cmulc<R>(v, w);
     }
     return v;
   }
 };
 
-template <typename R> struct GenOut {
+template <typename R, bool LEAN> struct GenOut {
   cplx<R>* __restrict__ base;
   int64_t es;
   int cnt;
@@ -193,37 +207,60 @@ template <typename R> struct GenOut {
   int64_t lt;  // the line's twiddle index
   int tw_shift, tw_dir;
   R scale;
-  bool cs;
+  bool ok, cs;
 
-  __device__ __forceinline__ void put(int i, cplx<R>* p, cplx<R> v) const {
-    if (i >= cnt) return;
-    if (mul) v = cmul<R>(v, __ldg(mul + i * ves));
+  // outputs e0 + r*st of a butterfly
+  template <int RAD> __device__ __forceinline__ void store(int e0, int st, cplx<R>* v) const {
+    if (LEAN && !ok) return;
+    auto here = [&](int r) { return LEAN || e0 + r * st < cnt; };
+    auto twiddle = [&](int r, cplx<R> w) {
+      v[r] = tw_dir < 0 ? cmul<R>(v[r], w) : cmulc<R>(v[r], w);
+    };
+    if (!LEAN && mul) {
+#pragma unroll
+      for (int r = 0; r < RAD; ++r)
+        if (here(r)) v[r] = cmul<R>(v[r], __ldg(mul + (e0 + r * st) * ves));
+    }
     if (tab) {
-      const cplx<R> w = __ldg(tab + i * tab_es);
-      v = tw_dir < 0 ? cmul<R>(v, w) : cmulc<R>(v, w);
-    } else if (tw_hi) {
-      const int64_t e = lt * (int64_t)i;
-      const cplx<R> w = cmul<R>(__ldg(tw_hi + (e >> tw_shift)),
-                                __ldg(tw_lo + (e & ((int64_t(1) << tw_shift) - 1))));
+      const cplx<R>* p = tab + e0 * tab_es;
+#pragma unroll
+      for (int r = 0; r < RAD; ++r)
+        if (here(r)) twiddle(r, __ldg(row_ptr<LEAN>(p, st * tab_es, r)));
+    } else if (!LEAN && tw_hi) {
+#pragma unroll
+      for (int r = 0; r < RAD; ++r)
+        if (here(r)) twiddle(r, root(e0 + r * st));
+    }
+    if (scale != R(1)) {
+#pragma unroll
+      for (int r = 0; r < RAD; ++r) v[r] = cscale<R>(v[r], scale);
+    }
+    cplx<R>* p = base + e0 * es;
+#pragma unroll
+    for (int r = 0; r < RAD; ++r)
+      if (here(r)) write(row_ptr<LEAN>(p, st * es, r), v[r]);
+  }
+  __device__ __forceinline__ void one(int i, cplx<R> v) const {
+    if (LEAN ? !ok : i >= cnt) return;
+    if (!LEAN && mul) v = cmul<R>(v, __ldg(mul + i * ves));
+    if (tab || (!LEAN && tw_hi)) {
+      const cplx<R> w = tab ? __ldg(tab + i * tab_es) : root(i);
       v = tw_dir < 0 ? cmul<R>(v, w) : cmulc<R>(v, w);
     }
     if (scale != R(1)) v = cscale<R>(v, scale);
+    write(base + i * es, v);
+  }
+  __device__ __forceinline__ cplx<R> root(int i) const {
+    const int64_t e = lt * (int64_t)i;
+    return cmul<R>(__ldg(tw_hi + (e >> tw_shift)),
+                   __ldg(tw_lo + (e & ((int64_t(1) << tw_shift) - 1))));
+  }
+  __device__ __forceinline__ void write(cplx<R>* p, cplx<R> v) const {
     if (cs)
       __stcs(p, v);
     else
       *p = v;
   }
-  // outputs e0 + r*st of a butterfly
-  template <int RAD> __device__ __forceinline__ void store(int e0, int st, const cplx<R>* v) const {
-    cplx<R>* p = base + e0 * es;
-    const int64_t step = st * es;
-#pragma unroll
-    for (int r = 0; r < RAD; ++r) {
-      put(e0 + r * st, p, v[r]);
-      p += step;
-    }
-  }
-  __device__ __forceinline__ void one(int i, cplx<R> v) const { put(i, base + i * es, v); }
 };
 
 // A line's I/O made from the launch's arguments and the block's per-line
@@ -231,28 +268,31 @@ template <typename R> struct GenOut {
 // would take 35 registers): lb holds five arrays of G -- offsets of the input
 // and output, first batch level, twiddle index, elements present on load and
 // (upper half) on store.
-template <typename R> struct LineCtx {
+template <typename R, bool LEAN> struct LineCtx {
   const LineArgs& a;
   const int64_t* lb;
-  __device__ __forceinline__ GenIn<R> input(int g) const {
+  __device__ __forceinline__ GenIn<R, LEAN> input(int g) const {
     typedef cplx<R> C;
     const int G = a.G;
     const bool tw = a.tw_on_load && a.tw_tab;
-    return GenIn<R>{(const C*)a.in + lb[g], a.ld.es, (int)lb[4 * G + g],
-                    a.ld.mul ? (const C*)a.ld.mul + lb[2 * G + g] * a.ld.vls : nullptr, a.ld.ves,
-                    tw ? (const C*)a.tw_tab + lb[3 * G + g] * a.tw_ls : nullptr, a.tw_es,
-                    a.tw_dir, a.plain_io != 0};
+    return GenIn<R, LEAN>{(const C*)a.in + lb[g], a.ld.es, (int)lb[4 * G + g],
+                          !LEAN && a.ld.mul ? (const C*)a.ld.mul + lb[2 * G + g] * a.ld.vls
+                                            : nullptr,
+                          a.ld.ves, tw ? (const C*)a.tw_tab + lb[3 * G + g] * a.tw_ls : nullptr,
+                          a.tw_es, a.tw_dir};
   }
-  __device__ __forceinline__ GenOut<R> output(int g) const {
+  __device__ __forceinline__ GenOut<R, LEAN> output(int g) const {
     typedef cplx<R> C;
     const int G = a.G;
     const int64_t lt = lb[3 * G + g];
     const bool tab = a.tw_tab && !a.tw_on_load;
-    return GenOut<R>{(C*)a.out + lb[G + g], a.st.es, (int)(lb[4 * G + g] >> 32),
-                     a.st.mul ? (const C*)a.st.mul + lb[2 * G + g] * a.st.vls : nullptr, a.st.ves,
-                     tab ? (const C*)a.tw_tab + lt * a.tw_ls : nullptr, a.tw_es,
-                     a.tw_N ? (const C*)a.tw_hi : nullptr, (const C*)a.tw_lo, lt, a.tw_shift,
-                     a.tw_dir, (R)a.scale, a.st_stream != 0};
+    const int cnt = (int)(lb[4 * G + g] >> 32);
+    return GenOut<R, LEAN>{(C*)a.out + lb[G + g], a.st.es, cnt,
+                           !LEAN && a.st.mul ? (const C*)a.st.mul + lb[2 * G + g] * a.st.vls
+                                             : nullptr,
+                           a.st.ves, tab ? (const C*)a.tw_tab + lt * a.tw_ls : nullptr, a.tw_es,
+                           !LEAN && a.tw_N ? (const C*)a.tw_hi : nullptr, (const C*)a.tw_lo, lt,
+                           a.tw_shift, a.tw_dir, (R)a.scale, cnt > 0, a.st_stream != 0};
   }
 };
 
@@ -272,13 +312,14 @@ __device__ __forceinline__ int mod_ns(int j, int Ns, Divisor d) {
 // values now stay in registers (see v below); before, every stage of every
 // program ran through 2.3 KB of local memory per thread, 2.6 times the
 // algorithmic traffic at 7168 points.  One B200, before -> after, same bits:
-// 23100 x 256 ComplexF32 (100 x 231) 178.6 -> 116.9 us, 176 x 1728 x 5
+// 23100 x 256 ComplexF32 (100 x 231) 178.6 -> 116.9 us (78.0 with the lean
+// form below), 176 x 1728 x 5
 // ComplexF64 158.1 -> 47.2, 6240 x 6 22.5 -> 16.4, irfft 648 x 189 x 46
 // 295.6 -> 224.2.
-template <typename R, int RAD, int DIR, int CAP>
+template <typename R, int RAD, int DIR, int CAP, bool LEAN>
 __device__ __forceinline__ void stage(cplx<R>* buf, int L, int Ns, Divisor nsd,
                                       const cplx<R>* __restrict__ tw, const R* pcs, int u, int T,
-                                      bool ld, bool st, const LineCtx<R>& io, int g) {
+                                      bool ld, bool st, const LineCtx<R, LEAN>& io, int g) {
   constexpr int UM = (RAD >= CAP) ? 1 : CAP / RAD;
   const int nb = L / RAD;
   // Defined for every butterfly, present or not: inside the loop over the
@@ -292,7 +333,7 @@ __device__ __forceinline__ void stage(cplx<R>* buf, int L, int Ns, Divisor nsd,
     for (int r = 0; r < RAD; ++r) v[q][r] = Sc<R>::mk(R(0), R(0));
   if (st) grid_release();
   if (ld) {
-    const GenIn<R> in = io.input(g);
+    const GenIn<R, LEAN> in = io.input(g);
 #pragma unroll
     for (int q = 0; q < UM; ++q) {
       const int j = u + q * T;
@@ -443,10 +484,10 @@ __device__ __forceinline__ int big_prime_offset(int P) {
 
 // The stages of program p.  ld: the first stage reads the line's input; st:
 // the last one writes its output; else the line is in `buf` before and after.
-template <typename R, int DIR, int CAP, bool BIG>
+template <typename R, int DIR, int CAP, bool BIG, bool LEAN>
 __device__ __forceinline__ void run_prog(cplx<R>* buf, const StageProg& p, const R* pcs, int u,
                                          int T, int* err, bool ld, bool st,
-                                         const LineCtx<R>& io, int g) {
+                                         const LineCtx<R, LEAN>& io, int g) {
   const cplx<R>* twb = (const cplx<R>*)p.tw;
   int Ns = 1, L = p.L;
 #pragma unroll 1
@@ -461,16 +502,16 @@ __device__ __forceinline__ void run_prog(cplx<R>* buf, const StageProg& p, const
     // values of this iteration.
     asm volatile("" : "+r"(u), "+r"(L));
     switch (rad) {
-      case 2: stage<R, 2, DIR, CAP>(buf, L, Ns, d, tw, pcs, u, T, l, t, io, g); break;
-      case 3: stage<R, 3, DIR, CAP>(buf, L, Ns, d, tw, pcs, u, T, l, t, io, g); break;
-      case 4: stage<R, 4, DIR, CAP>(buf, L, Ns, d, tw, pcs, u, T, l, t, io, g); break;
-      case 5: stage<R, 5, DIR, CAP>(buf, L, Ns, d, tw, pcs, u, T, l, t, io, g); break;
-      case 7: stage<R, 7, DIR, CAP>(buf, L, Ns, d, tw, pcs, u, T, l, t, io, g); break;
-      case 8: stage<R, 8, DIR, CAP>(buf, L, Ns, d, tw, pcs, u, T, l, t, io, g); break;
-      case 9: stage<R, 9, DIR, CAP>(buf, L, Ns, d, tw, pcs, u, T, l, t, io, g); break;
-      case 11: stage<R, 11, DIR, CAP>(buf, L, Ns, d, tw, pcs, u, T, l, t, io, g); break;
-      case 13: stage<R, 13, DIR, CAP>(buf, L, Ns, d, tw, pcs, u, T, l, t, io, g); break;
-      case 16: stage<R, 16, DIR, CAP>(buf, L, Ns, d, tw, pcs, u, T, l, t, io, g); break;
+      case 2: stage<R, 2, DIR, CAP, LEAN>(buf, L, Ns, d, tw, pcs, u, T, l, t, io, g); break;
+      case 3: stage<R, 3, DIR, CAP, LEAN>(buf, L, Ns, d, tw, pcs, u, T, l, t, io, g); break;
+      case 4: stage<R, 4, DIR, CAP, LEAN>(buf, L, Ns, d, tw, pcs, u, T, l, t, io, g); break;
+      case 5: stage<R, 5, DIR, CAP, LEAN>(buf, L, Ns, d, tw, pcs, u, T, l, t, io, g); break;
+      case 7: stage<R, 7, DIR, CAP, LEAN>(buf, L, Ns, d, tw, pcs, u, T, l, t, io, g); break;
+      case 8: stage<R, 8, DIR, CAP, LEAN>(buf, L, Ns, d, tw, pcs, u, T, l, t, io, g); break;
+      case 9: stage<R, 9, DIR, CAP, LEAN>(buf, L, Ns, d, tw, pcs, u, T, l, t, io, g); break;
+      case 11: stage<R, 11, DIR, CAP, LEAN>(buf, L, Ns, d, tw, pcs, u, T, l, t, io, g); break;
+      case 13: stage<R, 13, DIR, CAP, LEAN>(buf, L, Ns, d, tw, pcs, u, T, l, t, io, g); break;
+      case 16: stage<R, 16, DIR, CAP, LEAN>(buf, L, Ns, d, tw, pcs, u, T, l, t, io, g); break;
       default: {
         const int off = BIG ? big_prime_offset(rad) : -1;
         if (off >= 0) {
@@ -506,7 +547,7 @@ __device__ __forceinline__ void run_prog(cplx<R>* buf, const StageProg& p, const
 // each: 23100 x 256 ComplexF32 116.9 -> 102.8 us.
 constexpr int kIdle = 1 << 29;
 
-template <typename R, int CAP, bool BIG, bool OVERLAPPED>
+template <typename R, int CAP, bool BIG, bool LEAN, bool OVERLAPPED>
 __device__ __forceinline__ void line_body(const LineArgs& a, int64_t block, int u, int g, int tid,
                                           unsigned char* smraw) {
   // (OVERLAPPED: launched by launch_overlapped)
@@ -537,7 +578,7 @@ __device__ __forceinline__ void line_body(const LineArgs& a, int64_t block, int 
   }
   if constexpr (OVERLAPPED) grid_wait();
   __syncthreads();
-  const LineCtx<R> io{a, lb};
+  const LineCtx<R, LEAN> io{a, lb};
   // direct I/O: not for the prime stages, which work in shared memory, nor
   // for an empty program (a copy)
   const bool direct = a.prog.nst > 0;
@@ -548,12 +589,12 @@ __device__ __forceinline__ void line_body(const LineArgs& a, int64_t block, int 
   const int rad0 = direct ? a.prog.radix[0] : 1, nb0 = L / rad0;
   if (!ld) {
     if (a.ld.mode == 1) {  // (em) line fastest
-      const GenIn<R> src = io.input(g);
+      const GenIn<R, LEAN> src = io.input(g);
       for (int i = u; i < L; i += T) buf[padi(i)] = src.one(i, nb0, rad0);
     } else {               // element fastest, whatever the thread order
       const int gg = tid / T, uu = tid - gg * T;
       if (gg < G) {
-        const GenIn<R> src = io.input(gg);
+        const GenIn<R, LEAN> src = io.input(gg);
         C* d = sm + gg * Lp;
         for (int i = uu; i < L; i += T) d[padi(i)] = src.one(i, nb0, rad0);
       }
@@ -562,15 +603,15 @@ __device__ __forceinline__ void line_body(const LineArgs& a, int64_t block, int 
   }
   // One program, or (Bluestein) program -> pointwise multiply -> program in
   // the other direction.  The loop keeps one inlined copy per direction.
-  const int npass = a.mid ? 2 : 1;
+  const int npass = !LEAN && a.mid ? 2 : 1;
 #pragma unroll 1
   for (int ps = 0; ps < npass; ++ps) {
     const bool l = ld && ps == 0, t = st && ps == npass - 1;
     if ((ps == 0 ? a.dir1 : a.dir2) < 0)
-      run_prog<R, -1, CAP, BIG>(buf, a.prog, pcs, u, T, a.err, l, t, io, g);
+      run_prog<R, -1, CAP, BIG, LEAN>(buf, a.prog, pcs, u, T, a.err, l, t, io, g);
     else
-      run_prog<R, 1, CAP, BIG>(buf, a.prog, pcs, u, T, a.err, l, t, io, g);
-    if (ps == 0 && a.mid) {
+      run_prog<R, 1, CAP, BIG, LEAN>(buf, a.prog, pcs, u, T, a.err, l, t, io, g);
+    if (!LEAN && ps == 0 && a.mid) {
       const C* __restrict__ mid = (const C*)a.mid;
       const int64_t l0 = lb[2 * G + g];
       for (int k = u; k < L; k += T)
@@ -581,12 +622,12 @@ __device__ __forceinline__ void line_body(const LineArgs& a, int64_t block, int 
   if (!st) {
     grid_release();
     if (a.st.mode == 1 || !em) {
-      const GenOut<R> dst = io.output(g);
+      const GenOut<R, LEAN> dst = io.output(g);
       for (int i = u; i < L; i += T) dst.one(i, buf[padi(i)]);
     } else {
       const int gg = tid / T, uu = tid - gg * T;
       if (gg < G) {
-        const GenOut<R> dst = io.output(gg);
+        const GenOut<R, LEAN> dst = io.output(gg);
         const C* d = sm + gg * Lp;
         for (int i = uu; i < L; i += T) dst.one(i, d[padi(i)]);
       }
@@ -598,11 +639,11 @@ __device__ __forceinline__ void line_body(const LineArgs& a, int64_t block, int 
 template <typename R, int CAP, bool BIG> struct LineBounds {
   static constexpr int min_blocks = sizeof(R) == 4 && CAP == 16 && !BIG ? 2 : 1;
 };
-template <typename R, int CAP, bool BIG>
+template <typename R, int CAP, bool BIG, bool LEAN>
 __global__ void __launch_bounds__(512, LineBounds<R, CAP, BIG>::min_blocks) line_kernel(const __grid_constant__ LineArgs a) {
   extern __shared__ __align__(16) unsigned char smraw[];
   const int u = threadIdx.x, g = threadIdx.y;
-  line_body<R, CAP, BIG, true>(a, blockIdx.x, u, g, g * a.T + u, smraw);
+  line_body<R, CAP, BIG, LEAN, true>(a, blockIdx.x, u, g, g * a.T + u, smraw);
 }
 
 // Work-descriptor launch: many line transforms -- different lengths,
@@ -633,7 +674,7 @@ __global__ void __launch_bounds__(512, LineBounds<R, CAP, BIG>::min_blocks)
   const bool active = (int)threadIdx.x < nthr;
   const int u = active ? (int)threadIdx.x % sa.T : kIdle;
   const int g = active ? (int)threadIdx.x / sa.T : 0;
-  line_body<R, CAP, BIG, false>(sa, sblock, u, g, active ? (int)threadIdx.x : nthr, smraw);
+  line_body<R, CAP, BIG, false, false>(sa, sblock, u, g, active ? (int)threadIdx.x : nthr, smraw);
 }
 
 }  // namespace fb

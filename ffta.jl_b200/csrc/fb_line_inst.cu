@@ -9,22 +9,25 @@
 
 namespace fb {
 
-cudaError_t FB_LAUNCH(const LineArgs& a, size_t smem, cudaStream_t s) {
+template <bool LEAN>
+static cudaError_t launch_as(const LineArgs& a, size_t smem, cudaStream_t s) {
   static int set_bytes[64] = {0};
+  auto k = line_kernel<FB_R, FB_CAP, FB_BIG, LEAN>;
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   if (smem > 48 * 1024 && (dev >= 64 || set_bytes[dev] < (int)smem)) {
-    e = cudaFuncSetAttribute(line_kernel<FB_R, FB_CAP, FB_BIG>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     if (e != cudaSuccess) return e;
     if (dev < 64) set_bytes[dev] = 227 * 1024;
   }
   const int64_t nblk = (a.nlines + a.G - 1) / a.G;
   if (nblk <= 0) return cudaSuccess;
-  dim3 grid((unsigned)nblk), block(a.T, a.G);
-  return launch_overlapped(true, line_kernel<FB_R, FB_CAP, FB_BIG>, grid, block, smem, s,
+  return launch_overlapped(true, k, dim3((unsigned)nblk), dim3(a.T, a.G), smem, s,
                            with_divisors(a));
+}
+cudaError_t FB_LAUNCH(const LineArgs& a, size_t smem, cudaStream_t s) {
+  return a.plain_io && !a.mid ? launch_as<true>(a, smem, s) : launch_as<false>(a, smem, s);
 }
 
 // Launch ndesc descriptors (device arrays) as one grid of `nblocks` blocks of
