@@ -524,6 +524,32 @@ __global__ void __launch_bounds__(DirectBounds<R, T>::threads, DirectBounds<R, T
     gin = (const C*)a.ins[lo] + k * a.idist;
     gout = (C*)a.outs[lo] + k * a.odist;
   }
+  if constexpr (T == 1 && RL::n == 1) {
+    // One butterfly per thread: the threads' own loads and stores would be a
+    // line apart (32 L1 wavefronts a request), so packed lines go through
+    // shared memory: 16 x 200000 ComplexF32 29.6 -> 16.7 us (a copy takes 8).
+    constexpr int L = RL::r[0];
+    if (a.ndesc == 0 && a.idist == L && a.odist == L) {
+      const int64_t line0 = (int64_t)blockIdx.x * a.G, left = a.nlines - line0;
+      const int count = (int)(left < a.G ? left : a.G) * L;
+      C* sm = (C*)smraw;
+      const C* src = (const C*)a.in + line0 * L;
+      C* dst = (C*)a.out + line0 * L;
+      for (int i = threadIdx.y; i < count; i += a.G) sm[i / L * LPAD + i % L] = __ldcs(src + i);
+      __syncthreads();
+      C v[L];
+#pragma unroll
+      for (int r = 0; r < L; ++r) v[r] = buf[r];
+      butterfly<R, L, DIR>(v, (const R*)a.prime_cs);
+#pragma unroll
+      for (int r = 0; r < L; ++r) buf[r] = a.scale == 1.0 ? v[r] : cscale<R>(v[r], (R)a.scale);
+      __syncthreads();
+      grid_release();
+      for (int i = threadIdx.y; i < count; i += a.G)
+        store<R>(dst + i, sm[i / L * LPAD + i % L], a.st_stream != 0);
+      return;
+    }
+  }
   const DirectIn<R> in{gin, ok};
   const DirectOut<R> out{gout, ok, (R)a.scale, a.st_stream != 0};
   fast_prog<R, DIR, RL, T>(buf, in, out, (const C*)a.tw, (const R*)a.prime_cs, threadIdx.x);

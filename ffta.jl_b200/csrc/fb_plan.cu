@@ -658,6 +658,67 @@ static int tile_smem_cap(const FastFn* ff, int es) {
   return (int)std::max<size_t>(1, budget / ((size_t)(ff->lpad + 15) * es + 32));
 }
 
+static int pow2_floor(int v) {
+  int p = 1;
+  while (p * 2 <= v) p *= 2;
+  return p;
+}
+
+// Lines per block of a tile pass, at most `cap` by threads and shared memory.
+//
+// Neighbouring lines (em): a power of two, so that the rows of a block start
+// on sector boundaries and its warps divide evenly -- 16 ComplexF32 or 8
+// ComplexF64 lines (128-byte rows), twice that where those are fewer than 128
+// threads (19683 x 852 ComplexF64 pass 1, 9 threads: 8 lines 265 us, 16 lines
+// 254).  One B200, lines per block -> us: 27648 x 606 pass 1 (3 threads)
+// 170 -> 127, 32 -> 117; 23100 x 256 pass 1 (20 threads) 25 -> 97, 16 -> 92;
+// 2^16 x 16 pass 1 (16 threads) 32 -> 14.3, 16 -> 12.4.  A launch that runs in
+// one wave only with more lines keeps them (65537 x 16 pass 1: 14 lines 72.8,
+// 8 lines 76.7).
+//   A Bluestein middle pass takes 8 (65537 x 16: 9 -> 72.8, 8 -> 63.6; 27109
+// x 34: 10 -> 73.3, 8 -> 67.2).  A lean pass that also loads the four-step
+// twiddle, whose table loads add latency per line, takes 4 ComplexF32 or 2
+// ComplexF64 lines, at least 64 threads (2^20 x 16: 4 -> 139, 8 -> 147).
+//   Lines contiguous on load are spread over about four blocks per SM when
+// the batch is small, but never below a sector of neighbours on store (2^20 x
+// 1: 1 line 19.7, 4 lines 14.5; 2^18 x 1: 10.4, 8.0; 2^17 x 3 ComplexF64: 1
+// line 13.4, 2 lines 11.4).  Strided loads keep 64-byte rows.
+static int tile_lines(const LineArgs& a, const FastFn* ff, int es, int cap, bool em, int64_t nl) {
+  const int T = ff->T, sector = 32 / es;
+  if (a.mid) cap = std::min(cap, std::max(1, ff->mid_threads / T));
+  if (!em) {
+    int G = std::min(cap, std::max(1, 128 / T));
+    while (G > 1 && G / 2 >= nl) G /= 2;
+    if (a.ld.mode == 0)
+      while (G > 1 && nl / G < 4 * 148) G /= 2;
+    return G;
+  }
+  // ComplexF64 tiles of long lines: up to 4 lines (80 KB) rather than the 40
+  // KB budget's 2 (four-step columns of 1024: 0.37 -> 0.33 ms per N = 2^20 x
+  // 16 step)
+  if (es == 16 && cap < 4 && !a.mid) {
+    const int g80 = (int)((80 * 1024) / ((size_t)(ff->lpad + 15) * es + 32));
+    cap = std::max(cap, std::min(std::min(4, ff->tile_threads / T), g80));
+  }
+  int want = std::min(8 * sector, std::max(4 * sector, pow2_floor(std::max(1, 255 / T))));
+  if (a.mid) want = 8;
+  if (a.tw_on_load && a.plain_io) want = std::max(sector, pow2_floor(std::max(1, 127 / T)));
+  int G = pow2_floor(std::min(cap, want));
+  while (G > 1 && G / 2 >= nl) G /= 2;
+  if (a.ld.mode == 0) {
+    while (G > sector && nl / G < 4 * 148) G /= 2;
+  } else {
+    while (G > 2 * sector && nl / G < 148) G /= 2;
+    const auto waves = [&](int g) {
+      const int64_t fit = std::max(1, std::min(1024 / (g * T), (int)((227 * 1024) /
+                                   ((size_t)g * (ff->lpad + 15) * es + 1024))));
+      return ((nl + g - 1) / g + 148 * fit - 1) / (148 * fit);
+    };
+    if (cap > G && cap < 2 * G && waves(G) == 2 && waves(cap) == 1) G = cap;
+  }
+  return G;
+}
+
 // Switch a generic pass to the compile-time tile kernel of its length when
 // one is compiled (same arithmetic, direct HBM I/O, lines fastest across a
 // warp).  Bluestein passes need the forward-then-inverse order it implements.
@@ -686,30 +747,10 @@ static void use_tile(const fb_plan_s* P, Pass& p, const std::vector<int>& radice
   const int T = ff->T;
   const int thr_cap = tile_thread_cap(ff), smem_cap = tile_smem_cap(ff, es);
   const bool em = p.a.ld.mode == 1 || p.a.st.mode == 1;
-  // strided tiles: as many neighbouring lines as the block allows (longer
-  // contiguous runs per DRAM page); contiguous lines: 128-thread blocks
-  const int want = em ? thr_cap : std::max(1, 128 / T);
-  int G = std::min(std::min(thr_cap, smem_cap), want);
-  // ComplexF64 strided tiles of long lines: up to 4 lines (80 KB) rather
-  // than the 40 KB budget's 2 (four-step columns of 1024: 0.37 -> 0.33 ms
-  // per N = 2^20 x 16 step, autotuned); a lean pass that also loads the
-  // four-step twiddle takes half the lines (its table loads add latency
-  // per line: N = 2^20 C32 pass 2 and the short rows of 27648, 19683)
-  if (em && es == 16 && G < 4) {
-    const int g80 = (int)((80 * 1024) / ((size_t)(ff->lpad + 15) * es + 32));
-    G = std::max(G, std::min(std::min(4, thr_cap), g80));
-  }
-  if (em && p.a.tw_on_load && p.a.plain_io && G >= 4) G /= 2;
-  if (p.a.mid) G = std::min(G, std::max(1, ff->mid_threads / T));
   const int64_t nl = std::max<int64_t>(1, p.a.nlines);
-  while (G > 1 && G / 2 >= nl) G /= 2;
-  // lines contiguous on load: at least about four blocks per SM when the
-  // batch is small (strided loads keep their width for long DRAM runs)
-  if (p.a.ld.mode == 0)
-    while (G > 1 && nl / G < 4 * 148) G /= 2;
   p.staged = ff;
   p.a.T = T;
-  p.a.G = std::max(1, G);
+  p.a.G = std::max(1, tile_lines(p.a, ff, es, std::min(thr_cap, smem_cap), em, nl));
   if ((P->flags & FB_FLAG_TENSOR_STAGE) && ff->launch_tile_tc && p.a.plain_io) {
     // 512 threads per block: four 128-row tiles of the stage's GEMM
     p.tc = 1;
@@ -1137,10 +1178,12 @@ static Axis plan_direct_axis(fb_plan_s* P, int64_t n, LineX& x, int64_t is, int6
     p.fa.prime_cs = p.a.prime_cs;
     p.fa.scale = 1.0;
     const int es = elem_bytes(P->dtype);
-    // one line per block once a line fills a warp: measured faster than
-    // packing several lines into 256-thread blocks (fewer lines wait at each
-    // stage barrier); shorter lines share a block up to a warp's worth
-    int G = std::max(1, 32 / ff->T);
+    // one line per block from 64 threads: measured faster than packing
+    // several lines into 256-thread blocks (fewer lines wait at each stage
+    // barrier); shorter lines share a block up to 64 threads' worth (an SM
+    // holds at most 32 blocks; 243 x 8000 ComplexF32, 27 threads a line: one
+    // line 10.3 us, two 7.7), one-butterfly lines up to 128 (fast_direct_kernel)
+    int G = ff->T == 1 ? 128 : std::max(1, 64 / ff->T);
     while (G > 1 && (size_t)G * ff->lpad * es > 100 * 1024) G /= 2;
     while (G > 1 && G / 2 >= nl) G /= 2;
     p.fa.G = G;
