@@ -514,8 +514,11 @@ static bool make_line(int64_t n, int64_t cutoff, int dtype, LineX* x) {
 // length's kernels come to copy bandwidth: powers of two from 256 (radix-16
 // programs) 1.0, lines shorter than 16 2.0, others 1.25 -- measured on the
 // four-step splits of 27648: 1024 x 27 in 0.182 ms, 144 x 192 in 0.226 ms.
-// Cost factor of a four-step factor that has no compiled kernel.
-static const double kGenericPassCost = 3.0;
+// Cost factor of a four-step factor that has no compiled kernel.  One B200, 3
+// -> 1.5 -> 1 (us): 30030 x 100 ComplexF32 113.7 -> 45.4 -> 45.4, 20020 x 100
+// ComplexF64 79.7 -> 48.8 -> 48.9, 23100 x 256 78.2 -> 78.2 -> 102.1, 70000 x 60
+// 65.7 -> 65.7 -> 89.5.
+static const double kGenericPassCost = 1.5;
 
 static double line_cost(const LineX& x, bool weighted = false) {
   const double L = x.L;
@@ -1571,8 +1574,7 @@ static Axis plan_axis(fb_plan_s* P, int64_t n, int64_t is, int64_t os, std::vect
       if (prefer_split && (xa.kind != 0 || xb.kind != 0)) continue;
       const bool weighted = (n & (n - 1)) != 0;
       // a factor without a compiled kernel runs on the generic one, about
-      // three times slower per element (measured on configuration-5
-      // lengths: 200-600 GB/s against 1300-1900 GB/s); decided without
+      // half as fast again (kGenericPassCost); decided without
       // FB_FLAG_GENERIC_ONLY so that such plans keep the same split
       const auto gen = [&](const LineX& x) {
         return x.kind == 0 && !find_fast(P->dtype, x.L, x.radices) ? kGenericPassCost : 1.0;
