@@ -84,3 +84,21 @@ def test_real_data_aligned_to_one_real(dtype):
     torch.cuda.synchronize()
     assert rel(off.cpu().numpy() / n, x) <= 2 * bound
     assert float(buf[0]) == 0.0
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("batch", [1, 3, 33])
+@pytest.mark.parametrize("n", [64, 128, 256, 1024, 2048, 4096, 16384])
+def test_split_in_registers(n, batch, dtype):
+    """Halves whose last stage holds butterflies in pairs (j and n/2/radix - j)
+    split in registers: every output, and a line alone gives the same bits."""
+    import torch
+    rng = np.random.default_rng(n * 7 + batch)
+    x = rng.standard_normal((batch, n)).astype(dtype)
+    t = torch.from_numpy(x).cuda()
+    p = F.plan_rfft(t.T, 1)
+    assert "REAL-HALF(L=" in p.describe((n, batch)) and "complex plan" not in p.describe((n, batch))
+    y = (p * t.T).T
+    assert rel(y.cpu().numpy(), np.fft.rfft(x.astype(np.float64))) <= 4 * EPS[dtype] * np.log2(n)
+    one = t[batch // 2].clone()
+    assert torch.equal(F.plan_rfft(one) * one, y[batch // 2])
