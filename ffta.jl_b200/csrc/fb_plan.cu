@@ -2150,7 +2150,7 @@ static fb_plan_s* create_half_real_plan(int dtype, int dir, int rank, const int6
   for (int d = 0; d < rank; ++d) total *= dims[d];
   if (total <= 0) return nullptr;
   const int64_t L = n / 2;
-  if (L > INT32_MAX) return nullptr;
+  if (L >= INT32_MAX) return nullptr;  // k_real_half counts to L + 1 in 32 bits
   LineX x;
   const FastFn* ff = nullptr;
   if (make_direct(L, cutoff, dtype, &x) && x.kind == 0) {
