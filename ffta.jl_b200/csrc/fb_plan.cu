@@ -1589,6 +1589,13 @@ static Axis plan_axis(fb_plan_s* P, int64_t n, int64_t is, int64_t os, std::vect
       // the first pass's tiles narrow: 27648 = 27 x 1024 measured 0.141 ms
       // against 0.161 ms for 1024 x 27 (C32, 606 columns)
       if (is == 1 && b < 128 && a > b) c *= 1.25;
+      // ComplexF64 powers of two: every split has equal cost above, but a first
+      // factor of 256 (two radix-16 stages) saves a stage over 512 x 512 and 512 x
+      // 1024.  One B200, us: 2^18 x 32 130.9 -> 119.4, x 1 9.7 -> 9.6, 2^19 x 16
+      // 135.6 -> 123.9, x 1 15.9 -> 14.3.  Not with a second factor of 4096 (2^20
+      // x 8 143.5 -> 163.5), and not ComplexF32, whose large batches gain (2^18 x
+      // 64 130.1 -> 122.8) but single transforms lose (7.9 -> 10.2).
+      if (P->dtype == FB_C64 && !weighted && a == 256 && b >= 256 && b <= 2048) c *= 1.0 - 1e-6;
       if (c < best) {
         best = c;
         bN1 = a;
