@@ -2225,8 +2225,9 @@ static fb_plan_s* create_half_real_plan(int dtype, int dir, int rank, const int6
   P->in_span = P->real_kind == 1 ? total : half;
   P->out_span = P->real_kind == 1 ? half : total;
   // the split's twiddles w^k = exp(-2 pi i k / n)
-  void* wk = alloc_table(P.get(), (size_t)(L / 2 + 1) * elem_bytes(dtype));
-  cuda_check(gen_roots(dtype, wk, n, 1, L / 2 + 1, 0), "real split twiddles");
+  const int wt = ff ? dtype : FB_C64;  // k_real_half takes FP64 twiddles
+  void* wk = alloc_table(P.get(), (size_t)(L / 2 + 1) * elem_bytes(wt));
+  cuda_check(gen_roots(wt, wk, n, 1, L / 2 + 1, 0), "real split twiddles");
   RealArgs& a = P->ra;
   memset(&a, 0, sizeof(a));
   a.nlines = total / n;
