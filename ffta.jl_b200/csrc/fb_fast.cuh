@@ -166,6 +166,52 @@ template <typename R> struct DirectOut {
   }
 };
 
+// The L pairs of a real line (fast_real_kernel) that is aligned to one real
+// only: each value in two accesses.
+template <typename R> struct PairsIn {
+  const R* __restrict__ g;
+  bool ok;
+  template <int ST> struct Row {
+    const R* __restrict__ p;
+    bool ok;
+    __device__ __forceinline__ cplx<R> raw(int r) const {
+      return ok ? Sc<R>::mk(__ldcs(p + 2 * r * ST), __ldcs(p + 2 * r * ST + 1))
+                : Sc<R>::mk(R(0), R(0));
+    }
+    template <int RAD> __device__ __forceinline__ void fin(cplx<R>*) const {}
+  };
+  template <int ST> __device__ __forceinline__ Row<ST> at(int e0) const {
+    return Row<ST>{g + 2 * e0, ok};
+  }
+};
+template <typename R> struct PairsOut {
+  R* __restrict__ g;
+  bool ok;
+  R scale;
+  bool cs;
+  template <int ST> struct Row {
+    R* __restrict__ p;
+    bool ok;
+    R scale;
+    bool cs;
+    __device__ __forceinline__ void put(int r, cplx<R> v) const {
+      if (!ok) return;
+      if (scale != R(1)) v = cscale<R>(v, scale);
+      R* q = p + 2 * r * ST;
+      if (cs) {
+        __stcs(q, v.x);
+        __stcs(q + 1, v.y);
+      } else {
+        q[0] = v.x;
+        q[1] = v.y;
+      }
+    }
+  };
+  template <int ST> __device__ __forceinline__ Row<ST> at(int e0) const {
+    return Row<ST>{g + 2 * e0, ok, scale, cs};
+  }
+};
+
 // Full I/O (Bluestein and root-table passes).  Element i of a strided line,
 // present when i < cnt; the optional table `mul` (the chirp) is read at
 // mul + i*ves (the line's offset included), the twiddle on load
@@ -926,7 +972,9 @@ __device__ __forceinline__ void real_last_stage(const cplx<R>* buf, cplx<R>* o, 
   }
 }
 
-template <typename R, int DIR, class RL, int T>
+// ALIGNED: every real line starts at a multiple of a complex value, and is read
+// or written as such (one access per value); else PairsIn, PairsOut.
+template <typename R, int DIR, class RL, int T, bool ALIGNED>
 __global__ void __launch_bounds__(DirectBounds<R, T>::threads, DirectBounds<R, T>::min_blocks)
     fast_real_kernel(const RealArgs a) {
   typedef cplx<R> C;
@@ -946,11 +994,11 @@ __global__ void __launch_bounds__(DirectBounds<R, T>::threads, DirectBounds<R, T
   const bool cs = a.st_stream != 0;
   grid_wait();
   if constexpr (DIR < 0) {
-    const DirectIn<R> in{(const C*)((const R*)a.in + l * a.idist), ok};
+    typedef std::conditional_t<ALIGNED, DirectIn<R>, PairsIn<R>> In;
+    const In in{(decltype(In::g))((const R*)a.in + l * a.idist), ok};
     C* o = (C*)a.out + l * a.odist;
     if constexpr (real_in_registers<RL, T>()) {
-      fast_prog<R, -1, RL, T, DirectIn<R>, SmemIO, 0, false, RL::n - 1>(buf, in, SmemIO{}, tw, pcs,
-                                                                        u);
+      fast_prog<R, -1, RL, T, In, SmemIO, 0, false, RL::n - 1>(buf, in, SmemIO{}, tw, pcs, u);
       real_last_stage<R, RL, T>(buf, o, ok, tw, pcs, wk, sc, cs, u);
     } else {
       fast_prog<R, -1, RL, T>(buf, in, SmemIO{}, tw, pcs, u);
@@ -984,7 +1032,8 @@ __global__ void __launch_bounds__(DirectBounds<R, T>::threads, DirectBounds<R, T
       }
     }
     __syncthreads();
-    const DirectOut<R> out{(C*)((R*)a.out + l * a.odist), ok, sc, cs};
+    typedef std::conditional_t<ALIGNED, DirectOut<R>, PairsOut<R>> Out;
+    const Out out{(decltype(Out::g))((R*)a.out + l * a.odist), ok, sc, cs};
     fast_prog<R, 1, RL, T>(buf, SmemIO{}, out, tw, pcs, u);
   }
 }
@@ -1332,14 +1381,19 @@ template <typename R, class RL, int T> struct FastEntry {
       snprintf(g_launch_msg, sizeof(g_launch_msg), "no real kernel for L=%d", L);
       return cudaErrorNotSupported;
     } else {
-      static int set_fwd[64] = {0}, set_bwd[64] = {0};
+      static int set[4][64] = {{0}};
       const size_t smem = (size_t)a.G * LPAD * sizeof(cplx<R>);
-      auto k = dir < 0 ? fast_real_kernel<R, -1, RL, T> : fast_real_kernel<R, 1, RL, T>;
+      // (every line: they are an even number of reals apart)
+      const bool aligned = (uintptr_t)(dir < 0 ? a.in : a.out) % sizeof(cplx<R>) == 0;
+      auto k = dir < 0 ? (aligned ? fast_real_kernel<R, -1, RL, T, true>
+                                  : fast_real_kernel<R, -1, RL, T, false>)
+                       : (aligned ? fast_real_kernel<R, 1, RL, T, true>
+                                  : fast_real_kernel<R, 1, RL, T, false>);
       if (a.G < 1 || a.G * T > DirectBounds<R, T>::threads) {
         launch_failure(k, "real launch shape", L, T, a.G, smem, cudaErrorInvalidValue);
         return cudaErrorInvalidValue;
       }
-      cudaError_t e = configure(k, smem, dir < 0 ? set_fwd : set_bwd);
+      cudaError_t e = configure(k, smem, set[2 * (dir < 0) + aligned]);
       if (e != cudaSuccess) {
         launch_failure(k, "real smem attribute", L, T, a.G, smem, e);
         return e;
