@@ -509,17 +509,25 @@ static bool make_line(int64_t n, int64_t cutoff, int dtype, LineX* x) {
   return make_blue1(n, dtype, x);
 }
 
-// Relative cost of one line: work ~ L (log2 L + 4).  With `weighted` (splits
-// of lengths that are not powers of two) the work is scaled by how close the
-// length's kernels come to copy bandwidth: powers of two from 256 (radix-16
-// programs) 1.0, lines shorter than 16 2.0, others 1.25 -- measured on the
-// four-step splits of 27648: 1024 x 27 in 0.182 ms, 144 x 192 in 0.226 ms.
 // Cost factor of a four-step factor that has no compiled kernel.  One B200, 3
 // -> 1.5 -> 1 (us): 30030 x 100 ComplexF32 113.7 -> 45.4 -> 45.4, 20020 x 100
 // ComplexF64 79.7 -> 48.8 -> 48.9, 23100 x 256 78.2 -> 78.2 -> 102.1, 70000 x 60
 // 65.7 -> 65.7 -> 89.5.
 static const double kGenericPassCost = 1.5;
+// Cost of a prime stage of the generic kernel (stage_prime), per element and
+// unit of the prime: its work grows with the prime.  Every split into two
+// direct factors has the same primes; this decides between those and splits
+// that take a prime into a Bluestein factor.  One B200, 2^21 elements, without
+// this cost -> with it (us): 29252 ComplexF32 149.5 -> 66.5, 5871 108.0 -> 54.8,
+// 6142 ComplexF64 186.1 -> 118.0.  Of 5000 length-type pairs with a factor of
+// 17..71 it changes the split of 337; of 140 timed, none got slower.
+static const double kPrimeStageCost = 0.45;
 
+// Relative cost of one line: work ~ L (log2 L + 4).  With `weighted` (splits
+// of lengths that are not powers of two) the work is scaled by how close the
+// length's kernels come to copy bandwidth: powers of two from 256 (radix-16
+// programs) 1.0, lines shorter than 16 2.0, others 1.25 -- measured on the
+// four-step splits of 27648: 1024 x 27 in 0.182 ms, 144 x 192 in 0.226 ms.
 static double line_cost(const LineX& x, bool weighted = false) {
   const double L = x.L;
   const double c = L * (std::log2(std::max(2.0, L)) + 4.0);
@@ -1573,14 +1581,17 @@ static Axis plan_axis(fb_plan_s* P, int64_t n, int64_t is, int64_t os, std::vect
       if (!make_line(a, P->cutoff, P->dtype, &xa) || !make_line(b, P->cutoff, P->dtype, &xb)) continue;
       if (prefer_split && (xa.kind != 0 || xb.kind != 0)) continue;
       const bool weighted = (n & (n - 1)) != 0;
-      // a factor without a compiled kernel runs on the generic one, about
-      // half as fast again (kGenericPassCost); decided without
+      // what a factor without a compiled kernel costs on the generic one
+      // (kGenericPassCost, kPrimeStageCost); decided without
       // FB_FLAG_GENERIC_ONLY so that such plans keep the same split
-      const auto gen = [&](const LineX& x) {
-        return x.kind == 0 && !find_fast(P->dtype, x.L, x.radices) ? kGenericPassCost : 1.0;
+      const auto cost = [&](const LineX& x) {
+        const double c = line_cost(x, weighted);
+        if (x.kind != 0 || find_fast(P->dtype, x.L, x.radices)) return c;
+        double primes = 0;
+        for (int R : x.radices) primes += R > 16 ? R : 0;
+        return c * kGenericPassCost + kPrimeStageCost * primes * x.L;
       };
-      double c = line_cost(xa, weighted) * gen(xa) * (double)b +
-                 line_cost(xb, weighted) * gen(xb) * (double)a;
+      double c = cost(xa) * (double)b + cost(xb) * (double)a;
       // prefer balanced direct splits on ties, and the power-of-two factor
       // as the first pass (the strided columns)
       c *= 1.0 + 1e-9 * std::fabs(std::log((double)a) - std::log((double)b));
