@@ -520,7 +520,9 @@ static const double kGenericPassCost = 1.5;
 // that take a prime into a Bluestein factor.  One B200, 2^21 elements, without
 // this cost -> with it (us): 29252 ComplexF32 149.5 -> 66.5, 5871 108.0 -> 54.8,
 // 6142 ComplexF64 186.1 -> 118.0.  Of 5000 length-type pairs with a factor of
-// 17..71 it changes the split of 337; of 140 timed, none got slower.
+// 17..71 it changes the split of 337: to 0.76 of the time on average, of which
+// 32 to more (62620 ComplexF64 117.5 -> 156.7, a pad of 6561), and to no more
+// than 1.04 of the time before kGenericPassCost for any.
 static const double kPrimeStageCost = 0.45;
 
 // Relative cost of one line: work ~ L (log2 L + 4).  With `weighted` (splits
@@ -686,6 +688,11 @@ static int pow2_floor(int v) {
 // 2^16 x 16 pass 1 (16 threads) 32 -> 14.3, 16 -> 12.4.  A launch that runs in
 // one wave only with more lines keeps them (65537 x 16 pass 1: 14 lines 72.8,
 // 8 lines 76.7).
+//   Lines of up to 4 elements, one thread each, take 64: an SM holds at most 32
+// blocks, and 16 such lines a block left it 512 loads in flight (2^21 elements,
+// 16 lines -> 64: 13122 ComplexF64 pass 1 of length 2 105.7 -> 55.6, 8748, length
+// 4, 59.9 -> 35.8; ComplexF32, 32 -> 64: 4374 strided 54.3 -> 37.8; 128 lines:
+// 13122 52.0, 26244 ComplexF32 strided 57.4 against 46.3).
 //   A Bluestein middle pass takes 8 (65537 x 16: 9 -> 72.8, 8 -> 63.6; 27109
 // x 34: 10 -> 73.3, 8 -> 67.2).  A lean pass that also loads the four-step
 // twiddle, whose table loads add latency per line, takes 4 ComplexF32 or 2
@@ -712,6 +719,7 @@ static int tile_lines(const LineArgs& a, const FastFn* ff, int es, int cap, bool
     cap = std::max(cap, std::min(std::min(4, ff->tile_threads / T), g80));
   }
   int want = std::min(8 * sector, std::max(4 * sector, pow2_floor(std::max(1, 255 / T))));
+  if (a.prog.L <= 4) want = 64;
   if (a.mid) want = 8;
   if (a.tw_on_load && a.plain_io) want = std::max(sector, pow2_floor(std::max(1, 127 / T)));
   int G = pow2_floor(std::min(cap, want));
