@@ -583,9 +583,21 @@ __global__ void __launch_bounds__(DirectBounds<R, T>::threads, DirectBounds<R, T
       C* sm = (C*)smraw;
       const C* src = (const C*)a.in + line0 * L;
       C* dst = (C*)a.out + line0 * L;
-      for (int i = threadIdx.y; i < count; i += a.G) sm[i / L * LPAD + i % L] = __ldcs(src + i);
-      __syncthreads();
+      // count <= L * G.  Every load is issued before the first is used: 16 x 1000
+      // ComplexF64 3.2 us, in a loop of unknown length 5.3, with the threads' own
+      // loads 4.4 (16 x 200000 18.4, 32.0, 35.1).
       C v[L];
+#pragma unroll
+      for (int r = 0; r < L; ++r) {
+        const int i = threadIdx.y + r * a.G;
+        if (i < count) v[r] = __ldcs(src + i);
+      }
+#pragma unroll
+      for (int r = 0; r < L; ++r) {
+        const int i = threadIdx.y + r * a.G;
+        if (i < count) sm[i / L * LPAD + i % L] = v[r];
+      }
+      __syncthreads();
 #pragma unroll
       for (int r = 0; r < L; ++r) v[r] = buf[r];
       butterfly<R, L, DIR>(v, (const R*)a.prime_cs);
@@ -593,8 +605,11 @@ __global__ void __launch_bounds__(DirectBounds<R, T>::threads, DirectBounds<R, T
       for (int r = 0; r < L; ++r) buf[r] = a.scale == 1.0 ? v[r] : cscale<R>(v[r], (R)a.scale);
       __syncthreads();
       grid_release();
-      for (int i = threadIdx.y; i < count; i += a.G)
-        store<R>(dst + i, sm[i / L * LPAD + i % L], a.st_stream != 0);
+#pragma unroll
+      for (int r = 0; r < L; ++r) {
+        const int i = threadIdx.y + r * a.G;
+        if (i < count) store<R>(dst + i, sm[i / L * LPAD + i % L], a.st_stream != 0);
+      }
       return;
     }
   }
