@@ -1536,12 +1536,21 @@ template <typename R, class RL, int T> struct FastEntry {
     // middle pass of which more blocks fit an SM than its even share (449699
     // ComplexF64, 243 blocks, three fit: 75.8 us early, 64.2 not), and the rows
     // of a four-step where twice the even share fits (2^20 x 1 ComplexF32, 1024
-    // blocks of 64: 25.3 early, 19.6 not).  Lighter ones are bound by latency
-    // and start early (2^18 x 1, 512 blocks of 32: 10.4 early, 12.3 not; middle
-    // pass of 8761 x 3, 432 blocks of 8: 38.4 early, 40.9 not).
+    // blocks of 64: 25.3 early, 19.6 not).  So do ComplexF64 middle passes with
+    // 12 KB of lines to a block, 40 KB where the chirps are applied in the same
+    // pass: FP64 arithmetic is scarce per SM (184839 x 1, 365 blocks of 64 threads
+    // and 16 KB: 60.0 early, 43.1 not; 61441 x 2 59.8, 35.9; 5156 x 8, 32 blocks of
+    // 48 KB, 40.3, 25.1).  Lighter ones are bound by latency and start early (2^18
+    // x 1, 512 blocks of 32: 10.4 early, 12.3 not; middle passes of 8761 x 3, 432
+    // blocks of 8: 38.4, 40.9, of 73028 x 2 ComplexF32 37.6, 41.5, of 43913 x 2
+    // ComplexF64, 384 blocks of 8 KB, 33.4, 35.7, and of 2 x 971 ComplexF64, 32 KB
+    // with the chirps, 16.4, 18.9).
     bool early = true;
     const int64_t share = (nblk + kSms - 1) / kSms;
-    if ((mid || (a.plain_io && a.ld.mode == 0)) && share * a.G * T >= 256)
+    const size_t bytes = (size_t)a.G * L * sizeof(cplx<R>);
+    const bool heavy = share * a.G * T >= 256 ||
+                       (mid && sizeof(R) == 8 && bytes >= (a.ld.mul ? 40 : 12) * 1024);
+    if (heavy && (mid || (a.plain_io && a.ld.mode == 0)))
       early = (mid ? om : op).blocks(k, a.G * T, smem) < (mid ? share + 1 : 2 * share);
     e = launch_overlapped(early, k, dim3((unsigned)nblk), dim3(a.G, T),
                           smem, s, with_divisors(a));
