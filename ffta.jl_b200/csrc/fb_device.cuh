@@ -22,6 +22,12 @@ namespace fb {
 // us, 65537 x 16 81.4 -> 73.4, 4096 x 16384 206.4 -> 195.7, 2^16 x 1 10.3 ->
 // 8.1.
 //
+// What an earlier kernel of the stream may have written is read by ordinary
+// loads that stay behind grid_wait (__ldcs, bulk copies), never through the
+// read-only path (__ldg, const __restrict__): that one is for memory nobody
+// writes while the kernel is resident, which here begins before the previous
+// kernel has ended.  Tables are made once, ahead of the launches that read them.
+//
 // early = false: an ordinary launch.
 template <class... P, class... A>
 inline cudaError_t launch_overlapped(bool early, void (*k)(P...), dim3 grid, dim3 block,
@@ -43,8 +49,8 @@ inline cudaError_t launch_overlapped(bool early, void (*k)(P...), dim3 grid, dim
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // Let the stream's next kernel be launched once every block has come here (or
 // ended); it waits in its own grid_wait.  Called where a block begins its last
-// stage: released at their start, blocks of the next launch of less than a
-// wave crowded onto the SMs that this one left free (three-pass Bluestein
+// stage, after the loads of a program of one stage: released at their start,
+// blocks of the next launch of less than a wave crowded onto the SMs that this one left free (three-pass Bluestein
 // 449699 ComplexF64 61.4 -> 70.8 us).
 __device__ __forceinline__ void grid_release() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

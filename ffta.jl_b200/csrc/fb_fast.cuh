@@ -443,7 +443,7 @@ __device__ __forceinline__ void fast_stage(cplx<R>* buf, const In& in, const Out
   constexpr bool GOUT = S == RL::n - 1 && !std::is_same<Out, SmemIO>::value;
   static_assert(!TC || (S == 0 && RAD == 16 && UM == 1 && nb == T && std::is_same<R, float>::value),
                 "the tensor-core stage is a first radix-16 stage, one butterfly per thread");
-  if constexpr (GOUT) grid_release();
+  if constexpr (GOUT && !GIN) grid_release();
   cplx<R> v[UM][RAD];
 #pragma unroll
   for (int q = 0; q < UM; ++q) {
@@ -466,6 +466,7 @@ __device__ __forceinline__ void fast_stage(cplx<R>* buf, const In& in, const Out
       const int j = u + q * T;
       if (nb % T == 0 || j < nb) in.template at<nb>(j).template fin<RAD>(v[q]);
     }
+    if constexpr (GOUT) grid_release();
   }
   // in place: all reads of the line finish before any write, unless one side
   // is global memory

@@ -94,6 +94,8 @@ struct LineArgs {
   uint64_t wait_ns;     // limit of a wait on the block's own asynchronous
                         // work (tensor-core products); 0: kWaitNsDefault
   Divisor d0, d1;       // m0 and m1 (with_divisors; mul 0: divide in 64 bits)
+  int tables_fresh;     // 1: the stream's previous kernel wrote this one's tables
+                        // (the generic kernel then starts after its end)
 };
 
 // The launch's arguments with the reciprocals split_line divides by.

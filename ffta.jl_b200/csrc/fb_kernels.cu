@@ -306,6 +306,7 @@ cudaError_t convert_c64(int dtype, void* dst, const void* src_c64, int64_t n, do
 // fewer than 2^31 elements, in 64 bits beyond: with 64-bit divisions the
 // Hermitian extension of 648 x 189 x 46 ran at a seventh of memory speed (92
 // us); irfft 231 x 819 x 5 Float32 64.4 -> 53.3 us.
+// They are launched early (launch_overlapped): `in` is read by __ldcs alone.
 struct Dims {
   int rank;
   int64_t n[8];
@@ -343,37 +344,35 @@ struct RealGeom {
 };
 
 template <typename R>
-__global__ void k_real_to_complex(const R* __restrict__ in, cplx<R>* __restrict__ out,
-                                  int64_t count) {
+__global__ void k_real_to_complex(const R* in, cplx<R>* out, int64_t count) {
   grid_release();
   grid_wait();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < count;
        i += (int64_t)gridDim.x * blockDim.x)
-    out[i] = Sc<R>::mk(in[i], R(0));
+    out[i] = Sc<R>::mk(__ldcs(in + i), R(0));
 }
 
 template <typename R>
-__global__ void k_complex_to_real(const cplx<R>* __restrict__ in, R* __restrict__ out,
-                                  int64_t count) {
+__global__ void k_complex_to_real(const cplx<R>* in, R* out, int64_t count) {
   grid_release();
   grid_wait();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < count;
        i += (int64_t)gridDim.x * blockDim.x)
-    out[i] = in[i].x;
+    out[i] = __ldcs(in + i).x;
 }
 
 // out (dims with r0 cut to h) <- in (full dims): the first h entries along
 // r0; `half` holds (pre, h, post), n the full length along r0
 template <typename R>
-__global__ void k_extract_half(const cplx<R>* __restrict__ in, cplx<R>* __restrict__ out,
-                               Dims half, int64_t n, int64_t count) {
+__global__ void k_extract_half(const cplx<R>* in, cplx<R>* out, Dims half, int64_t n,
+                               int64_t count) {
   grid_release();
   grid_wait();
   for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < count;
        q += (int64_t)gridDim.x * blockDim.x) {
     int64_t t = q;
     const int64_t a = take_dim(half, 0, t), k = take_dim(half, 1, t);
-    out[q] = in[a + half.n[0] * (k + n * t)];
+    out[q] = __ldcs(in + (a + half.n[0] * (k + n * t)));
   }
 }
 
@@ -382,13 +381,12 @@ __global__ void k_extract_half(const cplx<R>* __restrict__ in, cplx<R>* __restri
 // (-k mod n) in every transformed dim), the symmetry of a real signal's
 // spectrum.
 template <typename R>
-__global__ void k_herm_extend(const cplx<R>* __restrict__ x, cplx<R>* __restrict__ z, RealGeom g,
-                              int64_t total) {
+__global__ void k_herm_extend(const cplx<R>* in, cplx<R>* z, RealGeom g, int64_t total) {
   grid_release();
   grid_wait();
   for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < total;
        q += (int64_t)gridDim.x * blockDim.x) {
-    // offsets of the entry itself and of its mirror image in x
+    // offsets of the entry itself and of its mirror image in `in`
     int64_t t = q, src = 0, mir = 0, stride = 1;
     bool mirror = false;
     for (int d = 0; d < g.dims.rank; ++d) {
@@ -399,7 +397,7 @@ __global__ void k_herm_extend(const cplx<R>* __restrict__ x, cplx<R>* __restrict
       mir += m * stride;
       stride *= d == g.r0 ? g.h : g.dims.n[d];
     }
-    const cplx<R> v = x[mirror ? mir : src];
+    const cplx<R> v = __ldcs(in + (mirror ? mir : src));
     z[q] = mirror ? Sc<R>::mk(v.x, -v.y) : v;
   }
 }
@@ -452,8 +450,8 @@ __device__ __forceinline__ double sum_products(Two<double> x, double p, Two<doub
 }
 template <typename R, bool SPLIT>
 __global__ void __launch_bounds__(256)
-    k_real_half(const cplx<R>* __restrict__ in, cplx<R>* __restrict__ out,
-                const double2* __restrict__ wk, int L, int64_t lines, R scale) {
+    k_real_half(const cplx<R>* in, cplx<R>* out, const double2* __restrict__ wk, int L,
+                int64_t lines, R scale) {
   typedef cplx<R> C;
   typedef Sc<R> S;
   grid_release();
@@ -571,7 +569,7 @@ cudaError_t herm_extend(int dtype, const void* x, void* z, int rank, const int64
 // out[sum_d k_d * os[d]] = in[sum_d k_d * is[d]] for every index (k_d < dims[d]):
 // a strided copy that moves an array between two layouts (rank <= 8).
 template <typename E>
-__global__ void k_permute(const E* __restrict__ in, E* __restrict__ out, PermCopy p, Dims dims) {
+__global__ void k_permute(const E* in, E* out, PermCopy p, Dims dims) {
   grid_release();
   grid_wait();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < p.count;
@@ -582,7 +580,7 @@ __global__ void k_permute(const E* __restrict__ in, E* __restrict__ out, PermCop
       oi += k * p.is[d];
       oo += k * p.os[d];
     }
-    out[oo] = in[oi];
+    out[oo] = __ldcs(in + oi);
   }
 }
 

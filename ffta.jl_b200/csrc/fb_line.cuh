@@ -331,7 +331,7 @@ __device__ __forceinline__ void stage(cplx<R>* buf, int L, int Ns, Divisor nsd,
   for (int q = 0; q < UM; ++q)
 #pragma unroll
     for (int r = 0; r < RAD; ++r) v[q][r] = Sc<R>::mk(R(0), R(0));
-  if (st) grid_release();
+  if (st && !ld) grid_release();
   if (ld) {
     const GenIn<R, LEAN> in = io.input(g);
 #pragma unroll
@@ -344,6 +344,7 @@ __device__ __forceinline__ void stage(cplx<R>* buf, int L, int Ns, Divisor nsd,
       const int j = u + q * T;
       if (j < nb) in.template finish<RAD>(j, nb, v[q]);
     }
+    if (st) grid_release();
   } else {
 #pragma unroll
     for (int q = 0; q < UM; ++q) {

@@ -23,7 +23,7 @@ static cudaError_t launch_as(const LineArgs& a, size_t smem, cudaStream_t s) {
   }
   const int64_t nblk = (a.nlines + a.G - 1) / a.G;
   if (nblk <= 0) return cudaSuccess;
-  return launch_overlapped(true, k, dim3((unsigned)nblk), dim3(a.T, a.G), smem, s,
+  return launch_overlapped(!a.tables_fresh, k, dim3((unsigned)nblk), dim3(a.T, a.G), smem, s,
                            with_divisors(a));
 }
 cudaError_t FB_LAUNCH(const LineArgs& a, size_t smem, cudaStream_t s) {

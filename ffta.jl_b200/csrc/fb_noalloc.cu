@@ -259,6 +259,7 @@ static int noalloc_run(const void* in, void* out, int64_t n, int64_t batch, int 
   a1.tw_lo = lo;
   a1.tw_hi = hi;
   a1.scale = 1.0;
+  a1.tables_fresh = 1;
   a1.T = T1;
   a1.G = std::max(1, std::min(16, line_max_threads() / T1));
   while (a1.G & (a1.G - 1)) --a1.G;  // element-major tiles need a power of two
