@@ -522,6 +522,9 @@ def _real_kind(x) -> str:
 def _col_major(x):
     """x as contiguous column-major memory (Julia layout) plus its dims."""
     if _is_torch(x):
+        # a lazily conjugated or negated view's storage is not its values, and
+        # contiguous() leaves it as it is where its layout is already right
+        x = x.resolve_conj().resolve_neg()
         perm = tuple(range(x.ndim - 1, -1, -1))
         return x.permute(perm).contiguous(), tuple(int(s) for s in x.shape)
     return np.asfortranarray(x), tuple(int(s) for s in x.shape)
