@@ -324,12 +324,11 @@ cudaError_t real_to_complex(int dtype, const void* in, void* out, int64_t count,
 cudaError_t complex_to_real(int dtype, const void* in, void* out, int64_t count, cudaStream_t s);
 cudaError_t extract_half(int dtype, const void* in, void* out, int64_t pre, int64_t n, int64_t h,
                          int64_t post, cudaStream_t s);
-// Half-length algorithm around a complex plan of length L: the split of
-// transformed lines (L complex values) into half spectra (L+1), or the merge
-// of half spectra into lines; wk[k] = exp(-i pi k / L), k <= L/2; `scale`
-// applies to the split.
-cudaError_t real_half(int dtype, bool split, const void* in, void* out, const void* wk, int L,
-                      int64_t lines, double scale, cudaStream_t s);
+// Half-length rfft around a complex plan of length L: the split of transformed
+// lines (L complex values) into half spectra (L+1), scaled; wk[k] = exp(-i pi k
+// / L) in FP64, k <= L/2.
+cudaError_t real_half(int dtype, const void* in, void* out, const void* wk, int L, int64_t lines,
+                      double scale, cudaStream_t s);
 cudaError_t herm_extend(int dtype, const void* x, void* z, int rank, const int64_t* dims, int r0,
                         int64_t h, uint32_t region, cudaStream_t s);
 

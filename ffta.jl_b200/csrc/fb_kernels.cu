@@ -402,17 +402,16 @@ __global__ void k_herm_extend(const cplx<R>* in, cplx<R>* z, RealGeom g, int64_t
   }
 }
 
-// The split and the merge of the half-length algorithm (fast_real_kernel's
-// formulas) as passes of their own, around a complex plan of length L = n/2
-// on the real line read as L complex values: for halves without a one-kernel
-// real transform.  Thread (k, line) handles the outputs k and L-k; a thread
-// keeps w^k for all its lines.  Bound by memory: one read and one write of
-// the half spectrum.  The full-length path these lengths took before (real
-// to complex, a transform of 2L points, extraction) moved 2.5 times as much.
+// The split of the half-length rfft (fast_real_kernel's formulas) as a pass of
+// its own, behind a complex plan of length L = n/2 on the real line read as L
+// complex values: for halves without a one-kernel real transform.  Thread (k,
+// line) handles the outputs k and L-k; a thread keeps w^k for all its lines.
+// Bound by memory: one read of the line and one write of the half spectrum.
+// The full-length path these lengths took before (real to complex, a transform
+// of 2L points, extraction) moved 2.5 times as much.
 // Each output is rounded about once, by double arithmetic and double w for
-// float data and by sums with their errors (Knuth's two-sum) for double data:
-// rounded at every operation, irfft 648 Float32 was 1.25e-7 from FP64 where
-// the full-length path is 1.03e-7.
+// float data and by sums with their errors (Knuth's two-sum) for double data,
+// so that what is left is the error of the transform of length L.
 template <typename R> struct Two;  // a sum of two reals, exact
 template <> struct Two<float> {
   double v;
@@ -448,10 +447,10 @@ __device__ __forceinline__ double sum_products(Two<double> x, double p, Two<doub
   e = __fma_rn(p, a.e, __fma_rn(q, b.e, e));
   return __dsub_rn(e, e) == 0.0 ? __dadd_rn(t.v, e) : t.v;  // infinities: e is not a number
 }
-template <typename R, bool SPLIT>
+template <typename R>
 __global__ void __launch_bounds__(256)
     k_real_half(const cplx<R>* in, cplx<R>* out, const double2* __restrict__ wk, int L,
-                int64_t lines, R scale) {
+                 int64_t lines, R scale) {
   typedef cplx<R> C;
   typedef Sc<R> S;
   grid_release();
@@ -461,47 +460,30 @@ __global__ void __launch_bounds__(256)
   const double2 w = __ldg(wk + k);
   for (int64_t l = blockIdx.y * (int64_t)blockDim.y + threadIdx.y; l < lines;
        l += (int64_t)gridDim.y * blockDim.y) {
-    if constexpr (SPLIT) {
-      const C* z = in + l * L;
-      C* o = out + l * (L + 1);
-      const C A = __ldcs(z + k);
-      if (k == 0) {
-        o[0] = S::mk(S::mul(S::add(A.x, A.y), scale), R(0));
-        o[L] = S::mk(S::mul(S::sub(A.x, A.y), scale), R(0));
-        continue;
-      }
-      const C B = __ldcs(z + (L - k));
-      // XX + w XY and conj(XX - w XY), with XX = (A + conj B)/2 and XY = -i (A -
-      // conj B)/2
-      const Two<R> xx = half_sum(A.x, B.x), xi = half_sum(A.y, -B.y);
-      const Two<R> yx = half_sum(B.y, A.y), yi = half_sum(B.x, -A.x);
-      o[k] = cscale<R>(S::mk(sum_products(xx, w.x, yx, -w.y, yi), sum_products(xi, w.x, yi, w.y, yx)),
-                       scale);
-      if (k != L - k)
-        o[L - k] = cscale<R>(S::mk(sum_products(xx, -w.x, yx, w.y, yi),
-                                   -sum_products(xi, -w.x, yi, -w.y, yx)), scale);
-    } else {
-      const C* y = in + l * (L + 1);
-      C* z = out + l * L;
-      const C A = __ldcs(y + k), B = __ldcs(y + (L - k));
-      if (k == 0) {
-        z[0] = S::mk(S::add(A.x, B.x), S::sub(A.x, B.x));
-        continue;
-      }
-      // XX + i conj(w) DD and conj(XX - i conj(w) DD), with XX = A + conj B and
-      // DD = A - conj B
-      const Two<R> xx = exact_sum(A.x, B.x), xi = exact_sum(A.y, -B.y);
-      const Two<R> dx = exact_sum(A.x, -B.x), di = exact_sum(A.y, B.y);
-      z[k] = S::mk(sum_products(xx, -w.x, di, w.y, dx), sum_products(xi, w.x, dx, w.y, di));
-      if (k != L - k)
-        z[L - k] = S::mk(sum_products(xx, w.x, di, -w.y, dx), -sum_products(xi, -w.x, dx, -w.y, di));
+    const C* z = in + l * L;
+    C* o = out + l * (L + 1);
+    const C A = __ldcs(z + k);
+    if (k == 0) {
+      o[0] = S::mk(S::mul(S::add(A.x, A.y), scale), R(0));
+      o[L] = S::mk(S::mul(S::sub(A.x, A.y), scale), R(0));
+      continue;
     }
+    const C B = __ldcs(z + (L - k));
+    // XX + w XY and conj(XX - w XY), with XX = (A + conj B)/2 and XY = -i (A -
+    // conj B)/2
+    const Two<R> xx = half_sum(A.x, B.x), xi = half_sum(A.y, -B.y);
+    const Two<R> yx = half_sum(B.y, A.y), yi = half_sum(B.x, -A.x);
+    o[k] = cscale<R>(S::mk(sum_products(xx, w.x, yx, -w.y, yi), sum_products(xi, w.x, yi, w.y, yx)),
+                     scale);
+    if (k != L - k)
+      o[L - k] = cscale<R>(S::mk(sum_products(xx, -w.x, yx, w.y, yi),
+                                 -sum_products(xi, -w.x, yi, -w.y, yx)), scale);
   }
 }
 
 template <typename R>
-static cudaError_t real_half_t(bool split, const void* in, void* out, const void* wk, int L,
-                               int64_t lines, double scale, cudaStream_t s) {
+static cudaError_t real_half_t(const void* in, void* out, const void* wk, int L, int64_t lines,
+                               double scale, cudaStream_t s) {
   typedef cplx<R> C;
   int tx = 1;
   while (tx < 256 && tx < L / 2 + 1) tx *= 2;
@@ -510,15 +492,14 @@ static cudaError_t real_half_t(bool split, const void* in, void* out, const void
   // about 16 blocks per SM in all: a thread of a long launch reuses its w^k
   const int64_t gy = std::min<int64_t>(std::min<int64_t>(want, 65535),
                                        std::max<int64_t>(1, 16 * 148 / gx));
-  auto k = split ? k_real_half<R, true> : k_real_half<R, false>;
-  return launch_overlapped(true, k, dim3((unsigned)gx, (unsigned)gy), block, 0, s, (const C*)in, (C*)out,
-                           (const double2*)wk, L, lines, (R)scale);
+  return launch_overlapped(true, k_real_half<R>, dim3((unsigned)gx, (unsigned)gy), block, 0, s,
+                           (const C*)in, (C*)out, (const double2*)wk, L, lines, (R)scale);
 }
-cudaError_t real_half(int dtype, bool split, const void* in, void* out, const void* wk, int L,
-                      int64_t lines, double scale, cudaStream_t s) {
+cudaError_t real_half(int dtype, const void* in, void* out, const void* wk, int L, int64_t lines,
+                      double scale, cudaStream_t s) {
   if (lines <= 0) return cudaSuccess;
-  return dtype == 0 ? real_half_t<float>(split, in, out, wk, L, lines, scale, s)
-                    : real_half_t<double>(split, in, out, wk, L, lines, scale, s);
+  return dtype == 0 ? real_half_t<float>(in, out, wk, L, lines, scale, s)
+                    : real_half_t<double>(in, out, wk, L, lines, scale, s);
 }
 
 cudaError_t real_to_complex(int dtype, const void* in, void* out, int64_t count, cudaStream_t s) {

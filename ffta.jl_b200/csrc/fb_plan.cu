@@ -622,9 +622,8 @@ struct fb_plan_s {
   // other region dims of the half array (or is null)
   const fb::FastFn* rfn = nullptr;
   fb::RealArgs ra;
-  // half-length real path of other halves L: a complex plan of length L on
-  // the real lines read as L complex values, the split or merge a pass of its
-  // own (hz: the lines between the two)
+  // rfft of other halves L: a complex plan of length L on the real lines read as
+  // L complex values, the split a pass of its own (hz: the lines between the two)
   std::unique_ptr<fb_plan_s> hplan;
   std::unique_ptr<fb::DevBuf> hz;
   // a strided region dim: the copies that bring it to the front and back
@@ -2150,13 +2149,59 @@ const char* fb_version(void) { return FB_VERSION; }
 // rounding.
 namespace fb {
 
+// The copies that bring a real plan's strided region dim (P->r0) to the front
+// and back, and the contiguous buffers between them.  P's dims, direction, r0
+// and rh are set; total and half are the elements of the real array and of the
+// half spectra.
+static void region_to_front(fb_plan_s* P, int64_t total, int64_t half) {
+  // dims in the order (r0, the others): contiguous lines
+  std::vector<int> perm{P->r0};
+  for (int d = 0; d < P->rank; ++d)
+    if (d != P->r0) perm.push_back(d);
+  std::vector<int64_t> hd(P->dims), st(P->rank), hst(P->rank);
+  hd[P->r0] = P->rh;
+  int64_t s = 1, hs = 1;
+  for (int d = 0; d < P->rank; ++d) {
+    st[d] = s;
+    hst[d] = hs;
+    s *= P->dims[d];
+    hs *= hd[d];
+  }
+  PermCopy full, hp;
+  memset(&full, 0, sizeof(full));
+  memset(&hp, 0, sizeof(hp));
+  full.rank = hp.rank = P->rank;
+  full.count = total;
+  hp.count = half;
+  int64_t cf = 1, ch = 1;
+  for (int d = 0; d < P->rank; ++d) {
+    full.dims[d] = P->dims[perm[d]];
+    hp.dims[d] = hd[perm[d]];
+    // real array: `st` (user layout) <-> contiguous (cf); half: hst <-> ch
+    full.is[d] = P->real_kind == 1 ? st[perm[d]] : cf;
+    full.os[d] = P->real_kind == 1 ? cf : st[perm[d]];
+    hp.is[d] = P->real_kind == 1 ? ch : hst[perm[d]];
+    hp.os[d] = P->real_kind == 1 ? hst[perm[d]] : ch;
+    cf *= full.dims[d];
+    ch *= hp.dims[d];
+  }
+  P->perm_full = full;
+  P->perm_half = hp;
+  P->zr.reset(new DevBuf((size_t)total * elem_bytes(P->dtype) / 2));
+  P->zc.reset(new DevBuf((size_t)half * elem_bytes(P->dtype)));
+}
+
 // FFTA's even-length real transform (src/plan.jl:398-442, :466-495): when
 // the first region dim is the contiguous one (dim 1) and has even length
 // n = 2L whose half runs on a specialised kernel, one fast_real_kernel pass
-// transforms every line at half length with the split fused in (other halves
-// run a complex plan of length L and a split pass, half the work and 0.4 of
-// the traffic of a transform of length n: rfft Float32 131072 x 4 24.6 ->
-// 18.0 us, irfft 648 x 189 x 46 226.9 -> 75.8, rfft 324 x 4545 36.9 -> 18.4),
+// transforms every line at half length with the split fused in (rfft of other
+// halves runs a complex plan of length L and a split pass, half the work and 0.4
+// of the traffic of a transform of length n: Float32 131072 x 4 24.6 -> 18.0 us,
+// 324 x 4545 36.9 -> 18.4; its error against FP64 is 0.95 to 1.05 of the
+// full-length one's in Float32, 1.00 on average over 95 lengths, and 0.79 to 1.09,
+// 1.01 on average, in Float64.  brfft of those halves stays at full length: there
+// the imaginary half of the transform's error is dropped, at half length none
+// of it is, and the error was 1.15 and 1.22 of that on average, up to 1.39),
 // and the other region dims (if any) are complex transforms of the n/2+1-long half
 // array -- after the real pass for rfft (in place on the output), before it
 // for brfft (input -> scratch).  Returns nullptr when the path does not apply.
@@ -2183,6 +2228,7 @@ static fb_plan_s* create_half_real_plan(int dtype, int dir, int rank, const int6
     ff = find_fast(dtype, (int)L, x.radices);
     if (ff && (!ff->launch_real || (int)ff->lpad != lpad_for((int)L))) ff = nullptr;
   }
+  if (!ff && dir == FB_BACKWARD) return nullptr;
   int ndev = 0;
   if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) {
     cudaGetLastError();
@@ -2213,34 +2259,7 @@ static fb_plan_s* create_half_real_plan(int dtype, int dir, int rank, const int6
   P->rh = L + 1;
   for (int r : region) P->region_mask |= 1u << r;
   const int64_t half = total / n * (L + 1);
-  if (r0 != 0) {
-    // dims in the order (r0, the others): the kernel's contiguous lines
-    std::vector<int> perm{r0};
-    for (int d = 0; d < rank; ++d)
-      if (d != r0) perm.push_back(d);
-    PermCopy full, hp;
-    memset(&full, 0, sizeof(full));
-    memset(&hp, 0, sizeof(hp));
-    full.rank = hp.rank = rank;
-    full.count = total;
-    hp.count = half;
-    int64_t cf = 1, ch = 1;
-    for (int d = 0; d < rank; ++d) {
-      full.dims[d] = dims[perm[d]];
-      hp.dims[d] = hd[perm[d]];
-      // real array: `st` (user layout) <-> contiguous (cf); half: hst <-> ch
-      full.is[d] = P->real_kind == 1 ? st[perm[d]] : cf;
-      full.os[d] = P->real_kind == 1 ? cf : st[perm[d]];
-      hp.is[d] = P->real_kind == 1 ? ch : hst[perm[d]];
-      hp.os[d] = P->real_kind == 1 ? hst[perm[d]] : ch;
-      cf *= full.dims[d];
-      ch *= hp.dims[d];
-    }
-    P->perm_full = full;
-    P->perm_half = hp;
-    P->zr.reset(new DevBuf((size_t)total * elem_bytes(dtype) / 2));
-    P->zc.reset(new DevBuf((size_t)half * elem_bytes(dtype)));
-  }
+  if (r0 != 0) region_to_front(P.get(), total, half);
   P->in_span = P->real_kind == 1 ? total : half;
   P->out_span = P->real_kind == 1 ? half : total;
   // the split's twiddles w^k = exp(-2 pi i k / n)
@@ -2256,7 +2275,7 @@ static fb_plan_s* create_half_real_plan(int dtype, int dir, int rank, const int6
   a.scale = 1.0;
   if (!ff) {
     const int64_t hdims[2] = {L, a.nlines}, hstr[2] = {1, L};
-    P->hplan.reset(create_plan(dtype, dir, 2, hdims, hstr, hstr, {0}, cutoff, flags));
+    P->hplan.reset(create_plan(dtype, FB_FORWARD, 2, hdims, hstr, hstr, {0}, cutoff, flags));
     P->hz.reset(new DevBuf((size_t)a.nlines * L * elem_bytes(dtype)));
   } else {
     // the length-L program
@@ -2294,8 +2313,21 @@ static fb_plan_s* create_real_plan(int dtype, int dir, int rank, const int64_t* 
     total *= dims[d];
   }
   if (auto* H = create_half_real_plan(dtype, dir, rank, dims, region, cutoff, flags)) return H;
-  std::unique_ptr<fb_plan_s> C(create_plan(dtype, dir, rank, dims, st.data(), st.data(), region,
-                                           cutoff, flags));
+  // brfft along one strided dim of even length: moved to the front and back, as
+  // on the half-length path, so that it gives the bits of a contiguous one
+  const bool front = dir == FB_BACKWARD && region.size() == 1 && region[0] != 0 && total > 0 &&
+                     dims[region[0]] % 2 == 0 && !(flags & FB_FLAG_GENERIC_ONLY);
+  std::vector<int64_t> cd(dims, dims + rank), cst(st);
+  if (front) {
+    std::rotate(cd.begin(), cd.begin() + region[0], cd.begin() + region[0] + 1);
+    int64_t s = 1;
+    for (int d = 0; d < rank; ++d) {
+      cst[d] = s;
+      s *= cd[d];
+    }
+  }
+  std::unique_ptr<fb_plan_s> C(create_plan(dtype, dir, rank, cd.data(), cst.data(), cst.data(),
+                                           front ? std::vector<int>{0} : region, cutoff, flags));
   std::unique_ptr<fb_plan_s> P(new fb_plan_s());
   P->dtype = dtype;
   P->dir = dir;
@@ -2316,41 +2348,31 @@ static fb_plan_s* create_real_plan(int dtype, int dir, int rank, const int64_t* 
   P->in_span = P->real_kind == 1 ? total : half;
   P->out_span = P->real_kind == 1 ? half : total;
   if (total > 0) P->zbuf.reset(new DevBuf((size_t)total * elem_bytes(dtype)));
+  if (front) region_to_front(P.get(), total, half);
   P->cplan = std::move(C);
   return P.release();
 }
 
 // The lines' real transform of a half-length plan (P->ra: in, out, scale and
-// store hint set): the one-kernel form, or the complex plan of length L and
-// the split or merge.  The complex plan reads and writes whole complex
-// values; real data that is aligned to one real only is copied through hz.
+// store hint set): the one-kernel form, or (rfft) the complex plan of length L
+// and the split.  The complex plan reads whole complex values; real data that
+// is aligned to one real only is copied through hz.
 static void real_lines(fb_plan_s* P, const RealArgs& a, cudaStream_t s) {
   if (P->rfn) {
     const cudaError_t e = P->rfn->launch_real(P->real_kind == 1 ? FB_FORWARD : FB_BACKWARD, a, s);
     if (e != cudaSuccess) cuda_check(e, last_launch_message());
     return;
   }
-  const size_t es = elem_bytes(P->dtype);
-  const int L = (int)(P->rh - 1);
   void* z = P->hz->p;
-  const auto aligned = [&](const void* p) { return reinterpret_cast<uintptr_t>(p) % es == 0; };
-  if (P->real_kind == 1) {
-    const void* src = a.in;
-    if (!aligned(src)) {
-      cuda_check(cudaMemcpyAsync(z, src, P->hz->bytes, cudaMemcpyDeviceToDevice, s), "real align");
-      src = z;
-    }
-    P->hplan->scale = 1.0;
-    execute_plan(P->hplan.get(), src, z, s);
-    cuda_check(real_half(P->dtype, true, z, a.out, a.wk, L, a.nlines, a.scale, s), "real split");
-  } else {
-    cuda_check(real_half(P->dtype, false, a.in, z, a.wk, L, a.nlines, 1.0, s), "real merge");
-    P->hplan->scale = a.scale;
-    void* dst = aligned(a.out) ? a.out : z;
-    execute_plan(P->hplan.get(), z, dst, s);
-    if (dst != a.out)
-      cuda_check(cudaMemcpyAsync(a.out, z, P->hz->bytes, cudaMemcpyDeviceToDevice, s), "real align");
+  const void* src = a.in;
+  if (reinterpret_cast<uintptr_t>(src) % elem_bytes(P->dtype) != 0) {
+    cuda_check(cudaMemcpyAsync(z, src, P->hz->bytes, cudaMemcpyDeviceToDevice, s), "real align");
+    src = z;
   }
+  P->hplan->scale = 1.0;
+  execute_plan(P->hplan.get(), src, z, s);
+  cuda_check(real_half(P->dtype, z, a.out, a.wk, (int)(P->rh - 1), a.nlines, a.scale, s),
+             "real split");
 }
 
 static void execute_real(fb_plan_s* P, const void* in, void* out, cudaStream_t s) {
@@ -2419,10 +2441,21 @@ static void execute_real(fb_plan_s* P, const void* in, void* out, cudaStream_t s
     execute_plan(P->cplan.get(), z, z, s);
     cuda_check(extract_half(P->dtype, z, out, pre, P->dims[P->r0], P->rh, post, s), "extract");
   } else {
-    cuda_check(herm_extend(P->dtype, in, z, P->rank, P->dims.data(), P->r0, P->rh,
-                           P->region_mask, s), "hermitian extension");
+    const int64_t* dims = P->dims.data();
+    const void* src = in;
+    void* dst = out;
+    if (P->zr) {  // a strided region dim, to the front and back
+      cuda_check(permute_copy(elem_bytes(P->dtype), in, P->zc->p, P->perm_half, s), "half gather");
+      dims = P->perm_full.dims;
+      src = P->zc->p;
+      dst = P->zr->p;
+    }
+    cuda_check(herm_extend(P->dtype, src, z, P->rank, dims, P->zr ? 0 : P->r0, P->rh,
+                           P->zr ? 1u : P->region_mask, s), "hermitian extension");
     execute_plan(P->cplan.get(), z, z, s);
-    cuda_check(complex_to_real(P->dtype, z, out, total, s), "complex to real");
+    cuda_check(complex_to_real(P->dtype, z, dst, total, s), "complex to real");
+    if (P->zr)
+      cuda_check(permute_copy(elem_bytes(P->dtype) / 2, dst, out, P->perm_full, s), "real scatter");
   }
 }
 
