@@ -111,7 +111,7 @@ struct GenSlots {
 // (absent ones load as zero and are not stored); `mul` (the chirp) is read
 // at mul + i*ves, the four-step twiddle at tab + i*tab_es, the line's offset
 // included in both.  LEAN (LineArgs::plain_io): every element present, no
-// chirp and no root tables, 32-bit strides; a twiddle on the loads is
+// chirp and no root tables, 32-bit steps between a butterfly's elements; a twiddle on the loads is
 // tw_elem's product instead of the entry itself.  What a pass rarely has is
 // applied to the registers in loops of its own, so the straight code between
 // loads and stores stays short: with the tests inside the unrolled loops a
@@ -119,14 +119,14 @@ struct GenSlots {
 // of 14 cycles per issue).  One B200, before -> after: 6240 x 6 ComplexF32 14.9
 // -> 10.6 us, 231 x 3000 11.4 -> 8.8, 176 x 1728 x 5 ComplexF64 40.9 -> 34.9,
 // irfft 260 x 66 27.2 -> 17.2.
-template <typename C> __device__ __forceinline__ C* step_ptr(C* p, int step, int r) {
+template <typename C> __device__ __forceinline__ C* step_ptr(C* p, uint32_t step, int r) {
   // p + r*step elements: a 32 x 32 -> 64 bit product added to the address
-  return (C*)((uintptr_t)p + (uint64_t)((int64_t)step * (int64_t)(r * (int)sizeof(C))));
+  return (C*)((uintptr_t)p + (uint64_t)step * (uint32_t)(r * (int)sizeof(C)));
 }
 template <bool LEAN, typename C>
 __device__ __forceinline__ C* row_ptr(C* p, int64_t step, int r) {
   if constexpr (LEAN)
-    return step_ptr(p, (int)step, r);
+    return step_ptr(p, (uint32_t)step, r);
   else
     return p + step * r;
 }
