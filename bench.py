@@ -15,6 +15,10 @@ larger than the 126 MB L2, so no flush is needed between steps.
   cpu_baseline  the oracle (C++ restatement of FFTA's algorithm) on the host's
             cores over a bounded sample of the same workload
 
+stdout has one line of JSON, the headline's; the other workloads' figures
+(configurations, serving, precision, real transforms, size sweep) are a line of
+JSON on stderr that begins with "bench details: ".
+
 `--impl reference` times FFTA's algorithm on the host cores (the oracle, as
 FFTA itself -- Julia -- is not installed) on the same metric.
 Multi-GPU: one process per GPU (torchrun), each transforming its own 16384
@@ -39,7 +43,8 @@ sys.path.insert(0, os.path.join(ROOT, "oracle"))
 N = 4096
 BATCH = 16384
 ES = 8  # bytes per ComplexF32
-# Other configurations, timed after the headline and reported under "extra":
+# Other configurations, timed after the headline and reported under "extra" in
+# the details:
 # (label, dtype, transform dims (Julia order), batch, region)
 EXTRA = [
     ("c64_n1024_b1", "c64", (1024,), 1),
@@ -209,6 +214,14 @@ def run_reference(args):
     }
     print(json.dumps(line))
     return 0
+
+
+def report(line, details):
+    """The result as one line of JSON on stdout, short enough for a reader that
+    keeps the end of the output; the other workloads' figures as one line on
+    stderr, ahead of it."""
+    print("bench details: " + json.dumps(details), file=sys.stderr, flush=True)
+    print(json.dumps(line), flush=True)
 
 
 def julia_probe():
@@ -715,13 +728,14 @@ def main():
             "gpu_launches": launches_per_step * args.steps,
             "clocks": clk.summary(),
             "cpu_baseline": cpu,
+        }
+        report(line, {
             "extra": extra,
             "serving": serving_out,
             "config4_precision": precision or None,
             "real_transforms": real_out or None,
             "reference_size_sweep": sweep_out or None,
-        }
-        print(json.dumps(line))
+        })
     if world > 1:
         dist.destroy_process_group()
     return 0
