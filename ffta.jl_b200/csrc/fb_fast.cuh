@@ -67,41 +67,24 @@ __host__ __device__ constexpr int lpad_of(int L) {
                                                : (L - 1) + ((L - 1) >> 4) + 2;
 }
 
-// Shared-memory slot of element e of a line.  Power-of-two strides would hit
-// the same banks, so even lengths skip one slot every 16 (padi); odd lengths
-// (powers of three and 5-smooth odd lengths) have only odd strides, which
-// spread over the banks by themselves, and are stored flat.
-template <class RL> __device__ __forceinline__ int pidx(int e) {
-  if constexpr (prog_len<RL>() % 2 == 1)
-    return e;
-  else
-    return padi(e);
-}
+// Whether a program's lines are stored flat (fb_internal.h, slot_of).
+template <class RL> __host__ __device__ constexpr bool flat() { return prog_len<RL>() % 2 == 1; }
+template <class RL> __device__ __forceinline__ int pidx(int e) { return slot_of(flat<RL>(), e); }
 
-// Slots of a butterfly's elements e0 + r*ST.  Where the pad of those elements
-// differs from e0's by a constant, the slot is pidx(e0) plus a compile-time
-// offset (one address per butterfly, immediate offsets in the accesses)
-// instead of an add, a shift and an add per element:
-//   reads  (ST = nb = L/RAD, e0 = j < nb): nb a multiple of 16, or a divisor
-//          of 16 (then j + (r*nb mod 16) < 16);
-//   writes (ST = Ns, e0 = M*Ns*RAD + k, k < Ns): Ns a multiple of 16, or a
-//          divisor of 16 with Ns*RAD a multiple or a divisor of 16.
-// In both cases (e0 + r*ST) >> 4 = (e0 >> 4) + ((r*ST) >> 4).  With the rows
-// of the I/O functors below and the 32-bit reciprocals of split_line, one B200,
-// before -> after, same bits: 2^20 x 16 ComplexF32 155.6 -> 147.7 us, 27648 x
-// 606 140.8 -> 134.6, 65537 x 16 (Bluestein) 94.1 -> 81.4, 4096 x 4096 2-D
-// 141.3 -> 137.3, rfft 4096 x 16384 128.2 -> 123.1; one-pass complex batches
-// are bound by memory and did not change.
-template <class RL, int RAD, int ST, bool WR> __host__ __device__ constexpr bool const_pad() {
-  return prog_len<RL>() % 2 == 1 || ST % 16 == 0 ||
-         (16 % ST == 0 && (!WR || (ST * RAD) % 16 == 0 || 16 % (ST * RAD) == 0));
-}
+// Slots of a butterfly's elements e0 + r*ST.  Where const_slots says so, the
+// slot is pidx(e0) plus a compile-time offset (one address per butterfly,
+// immediate offsets in the accesses) instead of an add, a shift and an add per
+// element.  With the rows of the I/O functors below and the 32-bit reciprocals
+// of split_line, one B200, before -> after, same bits: 2^20 x 16 ComplexF32 155.6
+// -> 147.7 us, 27648 x 606 140.8 -> 134.6, 65537 x 16 (Bluestein) 94.1 -> 81.4,
+// 4096 x 4096 2-D 141.3 -> 137.3, rfft 4096 x 16384 128.2 -> 123.1; one-pass
+// complex batches are bound by memory and did not change.
 template <class RL, int RAD, int ST, bool WR> struct Slots {
   int e0, p0;
   __device__ __forceinline__ explicit Slots(int e) : e0(e), p0(pidx<RL>(e)) {}
   __device__ __forceinline__ int operator[](int r) const {
-    if constexpr (const_pad<RL, RAD, ST, WR>())
-      return p0 + r * ST + (prog_len<RL>() % 2 == 1 ? 0 : (r * ST) >> 4);
+    if constexpr (const_slots(flat<RL>(), RAD, ST, WR))
+      return p0 + slot_step(flat<RL>(), r * ST);
     else
       return pidx<RL>(e0 + r * ST);
   }

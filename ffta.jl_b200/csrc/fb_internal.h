@@ -45,6 +45,38 @@ struct Divisor {
   uint32_t quot(uint32_t x) const { return (uint32_t)(((uint64_t)x * mul) >> shift); }
 };
 
+// Shared-memory slot of element e of a line.  Power-of-two strides would hit
+// the same banks, so even lengths skip one slot every 16 (padi); odd lengths
+// (powers of three and 5-smooth odd lengths) have only odd strides, which
+// spread over the banks by themselves, and the compiled kernels store them flat.
+#ifdef __CUDACC__
+#define FB_HD __host__ __device__ __forceinline__
+#else
+#define FB_HD inline
+#endif
+FB_HD constexpr int padi(int e) { return e + (e >> 4); }
+FB_HD constexpr int slot_of(bool flat, int e) { return flat ? e : padi(e); }
+// Whether the slots of a butterfly's elements e0 + r*st, r < rad, are e0's plus
+// slot_step(flat, r*st), whatever the butterfly:
+//   reads  (st = nb = L/rad, e0 = j < nb): nb a multiple of 16, or a divisor
+//          of 16 (then j + (r*nb mod 16) < 16);
+//   writes (st = Ns, e0 = M*Ns*rad + k, k < Ns): Ns a multiple of 16, or a
+//          divisor of 16 with Ns*rad a multiple or a divisor of 16.
+// In both cases (e0 + r*st) >> 4 = (e0 >> 4) + ((r*st) >> 4).
+FB_HD constexpr bool const_slots(bool flat, int rad, int st, bool write) {
+  return flat || st % 16 == 0 ||
+         (16 % st == 0 && (!write || (st * rad) % 16 == 0 || 16 % (st * rad) == 0));
+}
+FB_HD constexpr int slot_step(bool flat, int rst) { return rst + (flat ? 0 : rst >> 4); }
+// Slot of element e + r*st of a line of the generic kernel, held padded: padi(e)
+// = (17 e) >> 4, so the elements of a butterfly are one add, one shift and one
+// scaled add apart.
+struct GenSlots {
+  int e17, st17;
+  FB_HD GenSlots(int e, int st) : e17(17 * e), st17(17 * st) {}
+  FB_HD int operator[](int r) const { return (e17 + r * st17) >> 4; }
+};
+
 // A stage program: Stockham passes with the given radices, the per-stage
 // twiddle tables at tw + tw_off[s] (entries (r-1)*Ns + k = w_P^(r k),
 // P = Ns*R, forward sign).

@@ -26,8 +26,6 @@
 
 namespace fb {
 
-__host__ __device__ __forceinline__ int padi(int e) { return e + (e >> 4); }
-
 // Elements of a line that are present: i*ves + voff < vn, i.e. i < count.
 __device__ __forceinline__ int present_count(int64_t vn, int64_t ves, int64_t voff, bool ok) {
   if (!ok || voff >= vn) return 0;
@@ -97,14 +95,6 @@ __device__ __forceinline__ void butterfly(cplx<R>* v, const R* pcs) {
     dftp<R, DIR, RAD>(v, pcs + 2 * POff<RAD>::v);
   }
 }
-
-// Slot of element e + r*st of a line held padded: padi(e) = (17 e) >> 4, so
-// the elements of a butterfly are one add, one shift and one scaled add apart.
-struct GenSlots {
-  int e17, st17;
-  __device__ __forceinline__ GenSlots(int e, int st) : e17(17 * e), st17(17 * st) {}
-  __device__ __forceinline__ int operator[](int r) const { return (e17 + r * st17) >> 4; }
-};
 
 // ------------------------------------------------------------ I/O
 // One line's input or output in global memory.  `cnt` elements are present
