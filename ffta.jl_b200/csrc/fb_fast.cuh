@@ -322,12 +322,12 @@ __device__ __forceinline__ cplx<R> tw_mul(cplx<R> v, cplx<R> w, int tw_dir) {
 }
 template <typename R, int TW = kTwRuntime> struct PlainIn {
   const cplx<R>* __restrict__ base;
-  uint32_t es;
+  int es;
   const cplx<R>* tab;  // twiddle on load (LineArgs::tw_on_load)
   int tab_es, tw_dir;
   template <int ST> struct Row {
     const cplx<R>* p;
-    uint32_t step;
+    int step;
     const cplx<R>* pt;  // twiddle of element e0
     const cplx<R>* t0;  // the line's entry 0
     int tstep, dir;
@@ -358,13 +358,13 @@ template <typename R, int TW = kTwRuntime> struct PlainIn {
     }
   };
   template <int ST> __device__ __forceinline__ Row<ST> at(int e0) const {
-    return Row<ST>{base + (uint64_t)(uint32_t)e0 * es, es * ST, tab + (int64_t)e0 * tab_es, tab, tab_es * ST,
+    return Row<ST>{base + (int64_t)e0 * es, es * ST, tab + (int64_t)e0 * tab_es, tab, tab_es * ST,
                    tw_dir};
   }
 };
 template <typename R, int TW = kTwRuntime, bool SCALE = true> struct PlainOut {
   cplx<R>* __restrict__ base;
-  uint32_t es;
+  int es;
   const cplx<R>* tab;
   int tab_es, tw_dir;
   R scale;
@@ -372,7 +372,7 @@ template <typename R, int TW = kTwRuntime, bool SCALE = true> struct PlainOut {
   bool cs;
   template <int ST> struct Row {
     cplx<R>* p;
-    uint32_t step;
+    int step;
     const cplx<R>* pt;
     const cplx<R>* t0;
     int tstep, dir;
@@ -386,7 +386,7 @@ template <typename R, int TW = kTwRuntime, bool SCALE = true> struct PlainOut {
     }
   };
   template <int ST> __device__ __forceinline__ Row<ST> at(int e0) const {
-    return Row<ST>{base + (uint64_t)(uint32_t)e0 * es, es * ST, tab + (int64_t)e0 * tab_es, tab, tab_es * ST,
+    return Row<ST>{base + (int64_t)e0 * es, es * ST, tab + (int64_t)e0 * tab_es, tab, tab_es * ST,
                    tw_dir, scale, ok, cs};
   }
 };
@@ -804,7 +804,7 @@ __global__ void __launch_bounds__(TileThreads<R, T, MID>::value,
     const int64_t toff = lb[3 * G + g] * a.tw_ls;
     const C* ti = tin ? (st ? st : tin + toff) : nullptr;
     const C* to = tout ? (st ? st : tout + toff) : nullptr;
-    const uint32_t ies = (uint32_t)a.ld.es, oes = (uint32_t)a.st.es;
+    const int ies = (int)a.ld.es, oes = (int)a.st.es;
     const bool cs = a.st_stream != 0;
     // The lean passes of the four-step and 2-D schedules -- no twiddle, or a
     // twiddle on the loads or on the stores in the transform's direction,
@@ -1140,7 +1140,7 @@ __global__ void __launch_bounds__(TileThreads<R, T, false>::value,
     in.tab = tin ? tin + lt * a.tw_ls : nullptr;
     in.tab_es = (int)a.tw_es;
     in.tw_dir = a.tw_dir;
-    const PlainOut<R> out{(C*)a.out + q0 * a.st.s0 + q1 * a.st.s1 + q2 * a.st.s2, (uint32_t)a.st.es,
+    const PlainOut<R> out{(C*)a.out + q0 * a.st.s0 + q1 * a.st.s1 + q2 * a.st.s2, (int)a.st.es,
                           tout ? tout + lt * a.tw_ls : nullptr, (int)a.tw_es, a.tw_dir,
                           (R)a.scale, true,
                           a.st_stream != 0};
@@ -1243,9 +1243,9 @@ __global__ void __launch_bounds__(512, 2) fast_tc_tile_kernel(const LineArgs a) 
   const C* st = stage_twiddles<C>(a, lb + 3 * G, G, prog_len<RL>(), (C*)(slot + 2), g + G * u,
                                   G * T);
   const int tes = st ? 1 : (int)a.tw_es;
-  const PlainIn<float> in{(const C*)a.in + lb[G + g], (uint32_t)a.ld.es,
+  const PlainIn<float> in{(const C*)a.in + lb[G + g], (int)a.ld.es,
                           tin ? (st ? st : tin + lt * a.tw_ls) : nullptr, tes, a.tw_dir};
-  const PlainOut<float> out{(C*)a.out + lb[2 * G + g], (uint32_t)a.st.es,
+  const PlainOut<float> out{(C*)a.out + lb[2 * G + g], (int)a.st.es,
                             tout ? (st ? st : tout + lt * a.tw_ls) : nullptr, tes, a.tw_dir,
                             (float)a.scale, ok, a.st_stream != 0};
   const C* tw = (const C*)a.prog.tw;

@@ -109,14 +109,14 @@ __device__ __forceinline__ void butterfly(cplx<R>* v, const R* pcs) {
 // of 14 cycles per issue).  One B200, before -> after: 6240 x 6 ComplexF32 14.9
 // -> 10.6 us, 231 x 3000 11.4 -> 8.8, 176 x 1728 x 5 ComplexF64 40.9 -> 34.9,
 // irfft 260 x 66 27.2 -> 17.2.
-template <typename C> __device__ __forceinline__ C* step_ptr(C* p, uint32_t step, int r) {
+template <typename C> __device__ __forceinline__ C* step_ptr(C* p, int step, int r) {
   // p + r*step elements: a 32 x 32 -> 64 bit product added to the address
-  return (C*)((uintptr_t)p + (uint64_t)step * (uint32_t)(r * (int)sizeof(C)));
+  return (C*)((uintptr_t)p + (uint64_t)((int64_t)step * (int64_t)(r * (int)sizeof(C))));
 }
 template <bool LEAN, typename C>
 __device__ __forceinline__ C* row_ptr(C* p, int64_t step, int r) {
   if constexpr (LEAN)
-    return step_ptr(p, (uint32_t)step, r);
+    return step_ptr(p, (int)step, r);
   else
     return p + step * r;
 }

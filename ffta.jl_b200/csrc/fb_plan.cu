@@ -743,13 +743,13 @@ static int tile_lines(const LineArgs& a, const FastFn* ff, int es, int cap, bool
 static void use_tile(const fb_plan_s* P, Pass& p, const std::vector<int>& radices) {
   // The elements of a butterfly are L / R of the line's elements apart (R the
   // first radix on loads, the last on stores).  Those steps and the offsets in a
-  // twiddle table have 32 bits (31 in the tile kernel's full form, which also packs
-  // two batch indices into 64), all else has 64.  So lean passes take arrays of up to
-  // R * 34 GB of ComplexF32 (R * 69 GB of ComplexF64); those beyond (in place, over
-  // 69 GB with a radix 2 there, over 103 GB with a 3) run the generic kernel's
-  // full form.  One B200, line ends more than 2^31 elements apart, generic -> tile:
-  // 4096 strided x 524304 ComplexF32 39.6 -> 22.4 ms, 2187 x 2^20 29.8 -> 13.4,
-  // 2048 x 1048592 ComplexF64 35.2 -> 21.7.
+  // twiddle table are 32-bit and signed (the tile kernel's full form also packs two
+  // batch indices into 64 bits), all else has 64 bits.  So a strided pass takes arrays
+  // of up to R * 17 GB of ComplexF32 (R * 34 GB of ComplexF64); those beyond run the
+  // generic kernel's full form.  One B200, line ends more than 2^31 elements apart,
+  // generic -> tile: 4096 strided x 524304 ComplexF32 39.6 -> 22.4 ms, 2187 x 2^20
+  // 29.8 -> 13.4, 2048 x 1048592 ComplexF64 35.2 -> 21.7.  Unsigned steps would take
+  // twice the array and made the passes of 2^20 x 16 1.3 % slower.
   const int64_t L = p.a.prog.L, nst = p.a.prog.nst, bits31 = int64_t(1) << 31;
   const int64_t r0 = nst ? p.a.prog.radix[0] : 1, r1 = nst ? p.a.prog.radix[nst - 1] : 1;
   const int64_t step = std::max(p.a.ld.es * (L / r0), p.a.st.es * (L / r1));
@@ -759,7 +759,7 @@ static void use_tile(const fb_plan_s* P, Pass& p, const std::vector<int>& radice
   // lean pass is tw_elem's product in both kernels, so they keep equal bits.
   p.a.plain_io = !p.a.mid && !p.a.ld.mul && !p.a.st.mul && p.a.ld.vn == INT64_MAX &&
                  p.a.st.vn == INT64_MAX && !(p.a.tw_N && !p.a.tw_tab) && table &&
-                 step < 2 * bits31 && p.a.ld.count == L && p.a.st.count == L;
+                 step < bits31 && p.a.ld.count == L && p.a.st.count == L;
   if (P->flags & 1) return;
   if (!p.a.plain_io && !(table && step < bits31 && p.a.m0 < bits31 && p.a.m1 < bits31)) return;
   const FastFn* ff = find_fast(P->dtype, p.a.prog.L, radices);
