@@ -18,9 +18,9 @@ namespace fb {
 // kernel drains (programmatic stream serialization): the launch and the
 // block's index arithmetic overlap that kernel's end.  k must call
 // grid_wait() in every thread before it touches memory another kernel reads
-// or writes.  One B200, before -> after: 1000 x 1000 ComplexF32 18.4 -> 14.4
-// us, 65537 x 16 81.4 -> 73.4, 4096 x 16384 206.4 -> 195.7, 2^16 x 1 10.3 ->
-// 8.1.
+// or writes.  One B200, repeated buffers, before -> after: 1000 x 1000 ComplexF32
+// 18.4 -> 14.4 us, 65537 x 16 81.4 -> 73.4, 4096 x 16384 206.4 -> 195.7 (207 ->
+// 204 with inputs that change), 2^16 x 1 10.3 -> 8.1.
 //
 // What an earlier kernel of the stream may have written is read by ordinary
 // loads that stay behind grid_wait (__ldcs, bulk copies), never through the

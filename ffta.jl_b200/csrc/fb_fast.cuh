@@ -873,20 +873,6 @@ __global__ void __launch_bounds__(TileThreads<R, T, MID>::value,
 }
 
 // ------------------------------------------------------- real kernel
-// Half-length real transforms of contiguous lines of even length n = 2L, as
-// FFTA computes them (src/plan.jl:398-442 and :466-495, after Sorensen et
-// al.): rfft reads the real line as L complex values z[m] = x[2m] + i x[2m+1]
-// (no conversion pass), transforms them with the length-L program into
-// shared memory and splits Z into the n/2+1 outputs
-//   X[k]   = XX + w^k XY,  X[L-k] = conj(XX - w^k XY),
-//   XX = (Z[k] + conj Z[L-k]) / 2,  XY = i (conj Z[L-k] - Z[k]) / 2,
-//   X[0] = Re Z[0] + Im Z[0],  X[L] = Re Z[0] - Im Z[0],  w = exp(-2 pi i / n);
-// brfft builds Zb[k] = XX + i XY, Zb[L-k] = conj(XX - i XY) with
-// XX = Y[k] + conj Y[L-k], XY = w^-k (Y[k] - conj Y[L-k]) and
-// Zb[0] = (Re Y[0] + Re Y[L]) + i (Re Y[0] - Re Y[L]) in shared memory,
-// runs the inverse program and stores the L complex results as the 2L reals.
-// One HBM read and one write per element, as in the complex kernel, at half
-// its length.  w^k comes from a table computed in FP64 and rounded once.
 // One pair of rfft outputs from A = Z[k] and B = Z[L-k], 0 < k <= L/2.
 template <typename R>
 __device__ __forceinline__ void real_split(cplx<R>* o, int k, int L, cplx<R> A, cplx<R> B,
@@ -917,9 +903,10 @@ __device__ __forceinline__ void real_ends(cplx<R>* o, int L, cplx<R> z, R sc, bo
 // outputs, so a thread takes the butterflies in pairs: j and nb-j, and 0
 // with nb/2, which are their own partners.  Where a thread has an even number
 // of butterflies in that stage, the split then needs no trip of Z through
-// shared memory and no barrier.  Same operations as the loop over smem:
-// rfft 4096 x 16384 Float32 105.7 -> 93.7 us (a copy of these bytes 82), 4096 x
-// 4096 Float64 64.0 -> 54.2, 64 x 300000 56.4 -> 45.7.
+// shared memory and no barrier.  Same operations as the loop over smem; repeated
+// buffers: rfft 4096 x 16384 Float32 105.7 -> 93.7 us (111 with inputs that change;
+// a copy of these bytes 82), 4096 x 4096 Float64 64.0 -> 54.2, 64 x 300000 56.4
+// -> 45.7.
 template <class RL, int T> __host__ __device__ constexpr bool real_in_registers() {
   constexpr int RAD = RL::r[RL::n - 1], nb = prog_len<RL>() / RAD;
   return RL::n > 1 && RAD % 2 == 0 && nb % (2 * T) == 0;
@@ -971,6 +958,21 @@ __device__ __forceinline__ void real_last_stage(const cplx<R>* buf, cplx<R>* o, 
   }
 }
 
+// Half-length real transforms of contiguous lines of even length n = 2L, as
+// FFTA computes them (src/plan.jl:398-442 and :466-495, after Sorensen et
+// al.): rfft reads the real line as L complex values z[m] = x[2m] + i x[2m+1]
+// (no conversion pass), transforms them with the length-L program into
+// shared memory and splits Z into the n/2+1 outputs
+//   X[k]   = XX + w^k XY,  X[L-k] = conj(XX - w^k XY),
+//   XX = (Z[k] + conj Z[L-k]) / 2,  XY = i (conj Z[L-k] - Z[k]) / 2,
+//   X[0] = Re Z[0] + Im Z[0],  X[L] = Re Z[0] - Im Z[0],  w = exp(-2 pi i / n);
+// brfft builds Zb[k] = XX + i XY, Zb[L-k] = conj(XX - i XY) with
+// XX = Y[k] + conj Y[L-k], XY = w^-k (Y[k] - conj Y[L-k]) and
+// Zb[0] = (Re Y[0] + Re Y[L]) + i (Re Y[0] - Re Y[L]) in shared memory,
+// runs the inverse program and stores the L complex results as the 2L reals.
+// One HBM read and one write per element, as in the complex kernel, at half
+// its length.  w^k comes from a table computed in FP64 and rounded once.
+//
 // ALIGNED: every real line starts at a multiple of a complex value, and is read
 // or written as such (one access per value); else PairsIn, PairsOut.
 template <typename R, int DIR, class RL, int T, bool ALIGNED>
@@ -1288,8 +1290,6 @@ struct Occupancy {
   }
 };
 
-
-constexpr int kSms = 148;
 
 // Raise a kernel's dynamic shared-memory limit when a launch needs more than
 // the default 48 KB.  `set` is the caller's per-kernel, per-device record.

@@ -152,6 +152,8 @@ inline void set_stage_divisors(StageProg* p) {
   }
 }
 
+constexpr int kSms = 148;  // SMs of a B200
+
 // Output pairs of a radix >= 17 butterfly that one thread of the generic
 // kernel computes at most (stage_prime).
 constexpr int kPrimePairs = 16;

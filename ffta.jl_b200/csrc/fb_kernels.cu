@@ -491,7 +491,7 @@ static cudaError_t real_half_t(const void* in, void* out, const void* wk, int L,
   const int64_t gx = (L / 2 + 1 + tx - 1) / tx, want = (lines + block.y - 1) / block.y;
   // about 16 blocks per SM in all: a thread of a long launch reuses its w^k
   const int64_t gy = std::min<int64_t>(std::min<int64_t>(want, 65535),
-                                       std::max<int64_t>(1, 16 * 148 / gx));
+                                       std::max<int64_t>(1, 16 * kSms / gx));
   return launch_overlapped(true, k_real_half<R>, dim3((unsigned)gx, (unsigned)gy), block, 0, s,
                            (const C*)in, (C*)out, (const double2*)wk, L, lines, (R)scale);
 }

@@ -1,16 +1,21 @@
-// fb_kernels.cu -- the line kernel and the FP64 table generators.
+// fb_line.cuh -- the generic line kernel: any length with prime factors up to
+// 71, its radix program read at run time.
 //
-// A "line" is one 1-D transform of length L held in shared memory.  A block
-// holds G lines; each line is processed by T threads.  The kernel
-//   1. loads its lines (gathering strided elements, zero-filling absent ones,
-//      multiplying by an optional per-element table -- the Bluestein chirp),
-//   2. runs a Stockham stage program in shared memory (radix 2/3/4/5/8/16
-//      and odd-prime butterflies up to 71), in place: every stage reads its
+// A "line" is one 1-D transform of length L.  A block holds G lines; each line
+// is processed by T threads.  The kernel
+//   1. has its first stage read the line straight from global memory (gathering
+//      strided elements, zero-filling absent ones, multiplying by an optional
+//      per-element table -- the Bluestein chirp -- or the four-step twiddle); a
+//      first stage of a prime of 17 or more finds the line in shared memory,
+//   2. runs a Stockham stage program (radix 2/3/4/5/7/8/9/11/13/16 butterflies in
+//      registers, primes of 17 to 71 shared by the line's threads) that exchanges
+//      its values through shared memory, in place: every stage reads its
 //      butterflies into registers, synchronises, then writes,
 //   3. optionally multiplies by a pointwise table and runs a second program in
 //      the opposite direction (the Bluestein convolution in one kernel),
-//   4. stores, fusing the four-step twiddle, an optional per-element table
-//      and a scale factor.
+//   4. has its last stage store straight to global memory (a prime of 17 or more:
+//      from shared memory), fusing the four-step twiddle, an optional per-element
+//      table and a scale factor.
 // The same kernel serves batched 1-D columns, strided N-D axes, both passes
 // of the four-step and all three passes of the multi-pass Bluestein.
 //
@@ -107,8 +112,7 @@ __device__ __forceinline__ void butterfly(cplx<R>* v, const R* pcs) {
 // loads and stores stays short: with the tests inside the unrolled loops a
 // quarter of the kernel's stalls were instruction fetches (no_instruction 3.5
 // of 14 cycles per issue).  One B200, before -> after: 6240 x 6 ComplexF32 14.9
-// -> 10.6 us, 231 x 3000 11.4 -> 8.8, 176 x 1728 x 5 ComplexF64 40.9 -> 34.9,
-// irfft 260 x 66 27.2 -> 17.2.
+// -> 10.6 us, 231 x 3000 11.4 -> 8.8, 176 x 1728 x 5 ComplexF64 40.9 -> 34.9.
 template <typename C> __device__ __forceinline__ C* step_ptr(C* p, int step, int r) {
   // p + r*step elements: a 32 x 32 -> 64 bit product added to the address
   return (C*)((uintptr_t)p + (uint64_t)((int64_t)step * (int64_t)(r * (int)sizeof(C))));
@@ -536,12 +540,13 @@ __device__ __forceinline__ void run_prog(cplx<R>* buf, const StageProg& p, const
 // 32-byte sectors of each (pick_G); staging those loads through shared memory
 // instead formed the four-step twiddle element by element, 80 instructions
 // each: 23100 x 256 ComplexF32 116.9 -> 102.8 us.
+//
+// OVERLAPPED: launched by launch_overlapped.
 constexpr int kIdle = 1 << 29;
 
 template <typename R, int CAP, bool BIG, bool LEAN, bool OVERLAPPED>
 __device__ __forceinline__ void line_body(const LineArgs& a, int64_t block, int u, int g, int tid,
                                           unsigned char* smraw) {
-  // (OVERLAPPED: launched by launch_overlapped)
   typedef cplx<R> C;
   C* sm = (C*)smraw;
   const int T = a.T, G = a.G, L = a.prog.L;

@@ -653,7 +653,7 @@ struct fb_plan_s {
 
 namespace fb {
 
-static int pick_G(const fb_plan_s* P, int L, int T, int Lpad, bool elem_major, int64_t nlines,
+static int pick_G(const fb_plan_s* P, int T, int Lpad, bool elem_major, int64_t nlines,
                   bool mixed = false);
 static void apply_tuning(fb_plan_s* P);
 static void plan_tma(const fb_plan_s* P, Pass& p);
@@ -707,7 +707,7 @@ static int tile_lines(const LineArgs& a, const FastFn* ff, int es, int cap, bool
     int G = std::min(cap, std::max(1, 128 / T));
     while (G > 1 && G / 2 >= nl) G /= 2;
     if (a.ld.mode == 0)
-      while (G > 1 && nl / G < 4 * 148) G /= 2;
+      while (G > 1 && nl / G < 4 * kSms) G /= 2;
     return G;
   }
   // ComplexF64 tiles of long lines: up to 4 lines (80 KB) rather than the 40
@@ -724,13 +724,13 @@ static int tile_lines(const LineArgs& a, const FastFn* ff, int es, int cap, bool
   int G = pow2_floor(std::min(cap, want));
   while (G > 1 && G / 2 >= nl) G /= 2;
   if (a.ld.mode == 0) {
-    while (G > sector && nl / G < 4 * 148) G /= 2;
+    while (G > sector && nl / G < 4 * kSms) G /= 2;
   } else {
-    while (G > 2 * sector && nl / G < 148) G /= 2;
+    while (G > 2 * sector && nl / G < kSms) G /= 2;
     const auto waves = [&](int g) {
       const int64_t fit = std::max(1, std::min(1024 / (g * T), (int)((227 * 1024) /
                                    ((size_t)g * (ff->lpad + 15) * es + 1024))));
-      return ((nl + g - 1) / g + 148 * fit - 1) / (148 * fit);
+      return ((nl + g - 1) / g + kSms * fit - 1) / (kSms * fit);
     };
     if (cap > G && cap < 2 * G && waves(G) == 2 && waves(cap) == 1) G = cap;
   }
@@ -998,16 +998,19 @@ static void blue_tables(fb_plan_s* P, int64_t N, int64_t M, void** pre, void** p
   *mid = chirp_spectrum(P, N, M, 1.0);
 }
 
-// Lines per block of the generic kernel.  mixed: an element-major pass with one
+// Lines per block of the generic kernel: 100 KB of them, so that two blocks fit an
+// SM.  (The spread pitch of element-major lines and the 40 bytes a line has beside
+// it come on top: 2.2 KB at most where the 100 KB decide, at up to 16 lines;
+// line_smem_bytes has them all.)  mixed: an element-major pass with one
 // contiguous side, whose blocks take so many lines that a warp's 32/G
 // neighbouring elements of a line fill a 32-byte sector.
-static int pick_G(const fb_plan_s* P, int L, int T, int Lpad, bool elem_major, int64_t nlines,
+static int pick_G(const fb_plan_s* P, int T, int Lpad, bool elem_major, int64_t nlines,
                   bool mixed) {
   const int es = elem_bytes(P->dtype);
   const int thr_cap = std::max(1, std::max(line_max_threads(), T) / T);
   const size_t line_bytes = (size_t)Lpad * es + 24;
   const size_t budget = 100 * 1024;
-  int g_smem = (int)std::max<size_t>(1, budget / line_bytes);
+  const int g_smem = (int)std::max<size_t>(1, budget / line_bytes);
   int want = std::max(1, 256 / T);
   if (elem_major) want = std::max(want, es == 8 ? 16 : 8);
   int G = std::min(std::min(thr_cap, g_smem), want);
@@ -1019,7 +1022,6 @@ static int pick_G(const fb_plan_s* P, int L, int T, int Lpad, bool elem_major, i
     while (p * 2 <= G) p *= 2;
     G = p;
   }
-  (void)L;
   return std::max(1, G);
 }
 
@@ -1184,7 +1186,7 @@ static Axis plan_direct_axis(fb_plan_s* P, int64_t n, LineX& x, int64_t is, int6
   const bool st_em = os != 1 && !inner.empty() && inner[0].os == 1;
   p.a.ld.mode = ld_em ? 1 : 0;
   p.a.st.mode = st_em ? 1 : 0;
-  p.a.G = pick_G(P, x.L, x.T, p.a.Lpad, ld_em || st_em, nl, ld_em != st_em);
+  p.a.G = pick_G(P, x.T, p.a.Lpad, ld_em || st_em, nl, ld_em != st_em);
   ax.kind = x.kind == 0 ? "DIRECT" : "BLUE1";
   // Contiguous lines at one batch stride: the specialised direct-I/O kernel.
   const FastFn* ff = nullptr;
@@ -1340,8 +1342,8 @@ static Axis plan_four_axis(fb_plan_s* P, int64_t N, int64_t N1, int64_t N2, Line
     attach_twiddle(P, &p1.a, N, P->dir, N1, N2);
     p1.a.tw_level = tmode ? 1 : 0;
   }
-  p1.a.G = pick_G(P, x1.L, x1.T, p1.a.Lpad, true, p1.a.nlines);
-  p2.a.G = pick_G(P, x2.L, x2.T, p2.a.Lpad, p2.a.ld.mode == 1 || p2.a.st.mode == 1,
+  p1.a.G = pick_G(P, x1.T, p1.a.Lpad, true, p1.a.nlines);
+  p2.a.G = pick_G(P, x2.T, p2.a.Lpad, p2.a.ld.mode == 1 || p2.a.st.mode == 1,
                   p2.a.nlines, p2.a.ld.mode != p2.a.st.mode);
   std::ostringstream w1, w2;
   w1 << "FOUR" << (tmode ? "T" : "") << ".1(N1=" << N1 << (x1.kind ? " blue" : "")
@@ -1455,7 +1457,7 @@ static Axis plan_blue3_axis(fb_plan_s* P, int64_t N, int64_t is, int64_t os,
   if (!full_tw) attach_twiddle(P, &p1.a, M, FB_FORWARD, M1, M2, true);
   p1.a.ld.mode = is == 1 ? 1 : 0;
   p1.a.st.mode = 1;
-  p1.a.G = pick_G(P, x1.L, x1.T, p1.a.Lpad, true, p1.a.nlines);
+  p1.a.G = pick_G(P, x1.T, p1.a.Lpad, true, p1.a.nlines);
   // pass 2
   Pass p2;
   base_args(P, x2, &p2.a, FB_FORWARD);
@@ -1481,7 +1483,7 @@ static Axis plan_blue3_axis(fb_plan_s* P, int64_t N, int64_t is, int64_t os,
   }
   p2.a.ld.mode = 0;
   p2.a.st.mode = 1;
-  p2.a.G = pick_G(P, x2.L, x2.T, p2.a.Lpad, true, p2.a.nlines);
+  p2.a.G = pick_G(P, x2.T, p2.a.Lpad, true, p2.a.nlines);
   // pass 3
   Pass p3;
   base_args(P, x1, &p3.a, FB_BACKWARD);
@@ -1505,7 +1507,7 @@ static Axis plan_blue3_axis(fb_plan_s* P, int64_t N, int64_t is, int64_t os,
     attach_twiddle(P, &p3.a, M, FB_BACKWARD, M1, M2);
     p3.a.tw_on_load = 1;
   }
-  p3.a.G = pick_G(P, x1.L, x1.T, p3.a.Lpad, p3.a.st.mode == 1, p3.a.nlines);
+  p3.a.G = pick_G(P, x1.T, p3.a.Lpad, p3.a.st.mode == 1, p3.a.nlines);
   std::ostringstream w;
   w << "BLUE3(N=" << N << " M=" << M1 << "x" << M2 << ")";
   p1.what = w.str() + ".1";
