@@ -306,7 +306,9 @@ cudaError_t convert_c64(int dtype, void* dst, const void* src_c64, int64_t n, do
 // fewer than 2^31 elements, in 64 bits beyond: with 64-bit divisions the
 // Hermitian extension of 648 x 189 x 46 ran at a seventh of memory speed (92
 // us); irfft 231 x 819 x 5 Float32 64.4 -> 53.3 us.
-// They are launched early (launch_overlapped): `in` is read by __ldcs alone.
+// They are launched early (launch_overlapped): `in` is read by __ldcs alone, or by
+// __ldca where a sector or an element is read again (a strided copy, the mirror
+// image).
 struct Dims {
   int rank;
   int64_t n[8];
@@ -397,7 +399,7 @@ __global__ void k_herm_extend(const cplx<R>* in, cplx<R>* z, RealGeom g, int64_t
       mir += m * stride;
       stride *= d == g.r0 ? g.h : g.dims.n[d];
     }
-    const cplx<R> v = __ldcs(in + (mirror ? mir : src));
+    const cplx<R> v = __ldca(in + (mirror ? mir : src));
     z[q] = mirror ? Sc<R>::mk(v.x, -v.y) : v;
   }
 }
@@ -561,7 +563,7 @@ __global__ void k_permute(const E* in, E* out, PermCopy p, Dims dims) {
       oi += k * p.is[d];
       oo += k * p.os[d];
     }
-    out[oo] = __ldcs(in + oi);
+    out[oo] = __ldca(in + oi);
   }
 }
 
