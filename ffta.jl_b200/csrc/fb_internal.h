@@ -363,7 +363,10 @@ cudaError_t extract_half(int dtype, const void* in, void* out, int64_t pre, int6
 // / L) in FP64, k <= L/2.
 cudaError_t real_half(int dtype, const void* in, void* out, const void* wk, int L, int64_t lines,
                       double scale, cudaStream_t s);
-cudaError_t herm_extend(int dtype, const void* x, void* z, int rank, const int64_t* dims, int r0,
-                        int64_t h, uint32_t region, cudaStream_t s);
+// The real part of `in`, contiguous in the order of p's dims, to out + sum k_d*p.os[d].
+cudaError_t real_part(int dtype, const void* in, void* out, const PermCopy& p, cudaStream_t s);
+// x: half spectra of strides xs (dim r0 of length h); z: the full spectra, contiguous
+cudaError_t herm_extend(int dtype, const void* x, void* z, int rank, const int64_t* dims,
+                        const int64_t* xs, int r0, int64_t h, uint32_t region, cudaStream_t s);
 
 }  // namespace fb

@@ -340,6 +340,7 @@ __device__ __forceinline__ int64_t take_dim(const Dims& g, int i, int64_t& t) {
 }
 struct RealGeom {
   Dims dims;        // the full (complex) dims
+  int64_t xs[8];    // strides of the half spectra
   int r0;
   int64_t h;        // n/2 + 1 along r0
   uint32_t region;  // bit d: dim d is transformed
@@ -361,6 +362,19 @@ __global__ void k_complex_to_real(const cplx<R>* in, R* out, int64_t count) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < count;
        i += (int64_t)gridDim.x * blockDim.x)
     out[i] = __ldcs(in + i).x;
+}
+
+// out[sum_d k_d * os[d]] = the real part of in, contiguous in the order of dims
+template <typename R>
+__global__ void k_real_part(const cplx<R>* in, R* out, PermCopy p, Dims dims) {
+  grid_release();
+  grid_wait();
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < p.count;
+       i += (int64_t)gridDim.x * blockDim.x) {
+    int64_t t = i, oo = 0;
+    for (int d = 0; d < p.rank; ++d) oo += take_dim(dims, d, t) * p.os[d];
+    out[oo] = __ldcs(in + i).x;
+  }
 }
 
 // out (dims with r0 cut to h) <- in (full dims): the first h entries along
@@ -389,15 +403,14 @@ __global__ void k_herm_extend(const cplx<R>* in, cplx<R>* z, RealGeom g, int64_t
   for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < total;
        q += (int64_t)gridDim.x * blockDim.x) {
     // offsets of the entry itself and of its mirror image in `in`
-    int64_t t = q, src = 0, mir = 0, stride = 1;
+    int64_t t = q, src = 0, mir = 0;
     bool mirror = false;
     for (int d = 0; d < g.dims.rank; ++d) {
       const int64_t k = take_dim(g.dims, d, t);
       const int64_t m = ((g.region >> d) & 1) && k ? g.dims.n[d] - k : k;
       if (d == g.r0) mirror = k >= g.h;
-      src += k * stride;
-      mir += m * stride;
-      stride *= d == g.r0 ? g.h : g.dims.n[d];
+      src += k * g.xs[d];
+      mir += m * g.xs[d];
     }
     const cplx<R> v = __ldca(in + (mirror ? mir : src));
     z[q] = mirror ? Sc<R>::mk(v.x, -v.y) : v;
@@ -520,6 +533,15 @@ cudaError_t complex_to_real(int dtype, const void* in, void* out, int64_t count,
     return launch_overlapped(true, k_complex_to_real<double>, grid_for(count), 256, 0, s, (const double2*)in, (double*)out, count);
 }
 
+cudaError_t real_part(int dtype, const void* in, void* out, const PermCopy& p, cudaStream_t s) {
+  if (p.count <= 0) return cudaSuccess;
+  const Dims dims = make_dims(p.rank, p.dims);
+  if (dtype == 0)
+    return launch_overlapped(true, k_real_part<float>, grid_for(p.count), 256, 0, s, (const float2*)in, (float*)out, p, dims);
+  else
+    return launch_overlapped(true, k_real_part<double>, grid_for(p.count), 256, 0, s, (const double2*)in, (double*)out, p, dims);
+}
+
 cudaError_t extract_half(int dtype, const void* in, void* out, int64_t pre, int64_t n, int64_t h,
                          int64_t post, cudaStream_t s) {
   const int64_t count = pre * h * post;
@@ -532,11 +554,12 @@ cudaError_t extract_half(int dtype, const void* in, void* out, int64_t pre, int6
     return launch_overlapped(true, k_extract_half<double>, grid_for(count), 256, 0, s, (const double2*)in, (double2*)out, half, n, count);
 }
 
-cudaError_t herm_extend(int dtype, const void* x, void* z, int rank, const int64_t* dims, int r0,
-                        int64_t h, uint32_t region, cudaStream_t s) {
+cudaError_t herm_extend(int dtype, const void* x, void* z, int rank, const int64_t* dims,
+                        const int64_t* xs, int r0, int64_t h, uint32_t region, cudaStream_t s) {
   RealGeom g;
   memset(&g, 0, sizeof(g));
   g.dims = make_dims(rank, dims);
+  for (int d = 0; d < rank; ++d) g.xs[d] = xs[d];
   g.r0 = r0;
   g.h = h;
   g.region = region;

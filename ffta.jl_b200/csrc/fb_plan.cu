@@ -629,6 +629,8 @@ struct fb_plan_s {
   // a strided region dim: the copies that bring it to the front and back
   // (real array and half array) and the contiguous buffers between them
   fb::PermCopy perm_full, perm_half;
+  bool front = false;  // brfft at full length of a strided dim: the complex plan in
+                       // perm_full's order
   std::unique_ptr<fb::DevBuf> zr, zc;
   int r0 = 0;
   int64_t rh = 0;
@@ -2156,9 +2158,8 @@ const char* fb_version(void) { return FB_VERSION; }
 namespace fb {
 
 // The copies that bring a real plan's strided region dim (P->r0) to the front
-// and back, and the contiguous buffers between them.  P's dims, direction, r0
-// and rh are set; total and half are the elements of the real array and of the
-// half spectra.
+// and back.  P's dims, direction, r0 and rh are set; total and half are the
+// elements of the real array and of the half spectra.
 static void region_to_front(fb_plan_s* P, int64_t total, int64_t half) {
   // dims in the order (r0, the others): contiguous lines
   std::vector<int> perm{P->r0};
@@ -2193,8 +2194,6 @@ static void region_to_front(fb_plan_s* P, int64_t total, int64_t half) {
   }
   P->perm_full = full;
   P->perm_half = hp;
-  P->zr.reset(new DevBuf((size_t)total * elem_bytes(P->dtype) / 2));
-  P->zc.reset(new DevBuf((size_t)half * elem_bytes(P->dtype)));
 }
 
 // FFTA's even-length real transform (src/plan.jl:398-442, :466-495): when
@@ -2265,7 +2264,11 @@ static fb_plan_s* create_half_real_plan(int dtype, int dir, int rank, const int6
   P->rh = L + 1;
   for (int r : region) P->region_mask |= 1u << r;
   const int64_t half = total / n * (L + 1);
-  if (r0 != 0) region_to_front(P.get(), total, half);
+  if (r0 != 0) {
+    region_to_front(P.get(), total, half);
+    P->zr.reset(new DevBuf((size_t)total * elem_bytes(dtype) / 2));
+    P->zc.reset(new DevBuf((size_t)half * elem_bytes(dtype)));
+  }
   P->in_span = P->real_kind == 1 ? total : half;
   P->out_span = P->real_kind == 1 ? half : total;
   // the split's twiddles w^k = exp(-2 pi i k / n)
@@ -2319,8 +2322,9 @@ static fb_plan_s* create_real_plan(int dtype, int dir, int rank, const int64_t* 
     total *= dims[d];
   }
   if (auto* H = create_half_real_plan(dtype, dir, rank, dims, region, cutoff, flags)) return H;
-  // brfft along one strided dim of even length: moved to the front and back, as
-  // on the half-length path, so that it gives the bits of a contiguous one
+  // brfft along one strided dim of even length: the complex plan runs on
+  // contiguous lines, as on the half-length path, so that it gives the bits of a
+  // contiguous one; the extension and the real part read and write the strides
   const bool front = dir == FB_BACKWARD && region.size() == 1 && region[0] != 0 && total > 0 &&
                      dims[region[0]] % 2 == 0 && !(flags & FB_FLAG_GENERIC_ONLY);
   std::vector<int64_t> cd(dims, dims + rank), cst(st);
@@ -2354,6 +2358,7 @@ static fb_plan_s* create_real_plan(int dtype, int dir, int rank, const int64_t* 
   P->in_span = P->real_kind == 1 ? total : half;
   P->out_span = P->real_kind == 1 ? half : total;
   if (total > 0) P->zbuf.reset(new DevBuf((size_t)total * elem_bytes(dtype)));
+  P->front = front;
   if (front) region_to_front(P.get(), total, half);
   P->cplan = std::move(C);
   return P.release();
@@ -2447,21 +2452,22 @@ static void execute_real(fb_plan_s* P, const void* in, void* out, cudaStream_t s
     execute_plan(P->cplan.get(), z, z, s);
     cuda_check(extract_half(P->dtype, z, out, pre, P->dims[P->r0], P->rh, post, s), "extract");
   } else {
-    const int64_t* dims = P->dims.data();
-    const void* src = in;
-    void* dst = out;
-    if (P->zr) {  // a strided region dim, to the front and back
-      cuda_check(permute_copy(elem_bytes(P->dtype), in, P->zc->p, P->perm_half, s), "half gather");
-      dims = P->perm_full.dims;
-      src = P->zc->p;
-      dst = P->zr->p;
+    if (P->front) {
+      cuda_check(herm_extend(P->dtype, in, z, P->rank, P->perm_full.dims, P->perm_half.is, 0, P->rh,
+                             1u, s), "hermitian extension");
+      execute_plan(P->cplan.get(), z, z, s);
+      cuda_check(real_part(P->dtype, z, out, P->perm_full, s), "real part");
+      return;
     }
-    cuda_check(herm_extend(P->dtype, src, z, P->rank, dims, P->zr ? 0 : P->r0, P->rh,
-                           P->zr ? 1u : P->region_mask, s), "hermitian extension");
+    int64_t xs[8], stride = 1;
+    for (int d = 0; d < P->rank; ++d) {
+      xs[d] = stride;
+      stride *= d == P->r0 ? P->rh : P->dims[d];
+    }
+    cuda_check(herm_extend(P->dtype, in, z, P->rank, P->dims.data(), xs, P->r0, P->rh,
+                           P->region_mask, s), "hermitian extension");
     execute_plan(P->cplan.get(), z, z, s);
-    cuda_check(complex_to_real(P->dtype, z, dst, total, s), "complex to real");
-    if (P->zr)
-      cuda_check(permute_copy(elem_bytes(P->dtype) / 2, dst, out, P->perm_full, s), "real scatter");
+    cuda_check(complex_to_real(P->dtype, z, out, total, s), "complex to real");
   }
 }
 

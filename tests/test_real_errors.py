@@ -82,3 +82,24 @@ def test_infinities_and_nans(dtype):
     assert np.isposinf(y[3, 1].real) and not np.isnan(y[3, 1].imag)
     one = t[5].clone()
     assert np.array_equal(y[5], (F.plan_rfft(one) * one).cpu().numpy())
+
+
+# a first, a middle and a last strided dimension of three: the extension reads and
+# the real part writes the strides
+@pytest.mark.parametrize("dtype", [np.float32, np.float64])
+@pytest.mark.parametrize("n", [14, 324, 2018])
+@pytest.mark.parametrize("dim", [2, 3])
+def test_inverse_of_a_strided_dimension_of_three(dim, n, dtype):
+    import torch
+    shape = [3, 4, 5]  # Julia dims
+    shape[dim - 1] = n // 2 + 1
+    rng = np.random.default_rng(n + dim)
+    h = rng.standard_normal((2, *shape))
+    x = torch.from_numpy((h[0] + 1j * h[1]).astype(CPLX[dtype])).cuda()
+    x = x.permute(2, 1, 0).contiguous().permute(2, 1, 0)  # column-major memory
+    z = F.plan_irfft(x, n, dim) * x
+    lines = x.movedim(dim - 1, 0).reshape(n // 2 + 1, -1).T.contiguous()  # one row a line
+    want = (F.plan_irfft(lines.T, n, 1) * lines.T).T
+    assert torch.equal(z.movedim(dim - 1, 0).reshape(n, -1).T, want)
+    ld = np.fft.irfft(lines.cpu().numpy().astype(np.clongdouble), n=n)
+    assert err(want.cpu().numpy(), ld) <= 4 * np.finfo(dtype).eps * np.log2(n)
